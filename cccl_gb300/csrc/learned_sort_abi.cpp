@@ -170,6 +170,11 @@ CCCL_GB300_API CUresult cccl_gb300_learned_sort_build(
       ks.onesweep_first         = get_kernel(r.radix_library, nm.onesweep_first);
       ks.onesweep_dyn           = get_kernel(r.radix_library, nm.onesweep_dyn);
       ks.single_tile            = get_kernel(r.radix_library, nm.single_tile);
+      if (pol.finish == 1)
+      {
+        ks.finish      = get_kernel(r.radix_library, nm.finish);
+        ks.finish_tail = get_kernel(r.radix_library, nm.finish_tail);
+      }
     };
     radix(int(vb), kind, s->plain_pol, s->plain_ks);
     radix(0, KIND_UNSIGNED, s->sample_pol, s->sample_ks);

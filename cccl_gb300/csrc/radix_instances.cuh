@@ -83,6 +83,28 @@
   GB300_HISTOGRAM(KB, FP, SUF)         \
   GB300_MERGE_ALL_VALUES(KB, FP, SUF)
 
+// Partition and finish: whole 4- and 8-byte keys (finish_supported).
+#define GB300_FINISH(KB, VB, FP, SUF)                                                                             \
+  extern "C" __global__ void __launch_bounds__(gb300::finish_tpb(KB, VB, false) + 32, gb300::finish_minb(false))  \
+    gb300_finish_k##KB##_v##VB##_##SUF(const gb300::FinishParams p)                                               \
+  {                                                                                                               \
+    gb300::finish_body<KB, VB, FP, false>(p);                                                                     \
+  }                                                                                                               \
+  extern "C" __global__ void __launch_bounds__(gb300::finish_tpb(KB, VB, true) + 32, gb300::finish_minb(true))    \
+    gb300_finish_tail_k##KB##_v##VB##_##SUF(const gb300::FinishParams p)                                          \
+  {                                                                                                               \
+    if (gb300::gate_open(p.gate) && __ldcg(&p.ctrl->route) != 0u)                                                 \
+    {                                                                                                             \
+      gb300::finish_body<KB, VB, FP, true>(p);                                                                    \
+      gb300::finish_rest_body<KB, VB, FP>(p);                                                                     \
+    }                                                                                                             \
+  }
+
+#define GB300_FINISH_ALL(KB, FP, SUF)                                                                             \
+  GB300_FINISH(KB, 0, FP, SUF)                                                                                    \
+  GB300_FINISH(KB, 4, FP, SUF)                                                                                    \
+  GB300_FINISH(KB, 8, FP, SUF)
+
 extern "C" __global__ void __launch_bounds__(256) gb300_init(const gb300::InitParams p)
 {
   gb300::init_body(p);

@@ -23,6 +23,7 @@
 //    so no memset runs between passes.
 #pragma once
 
+#include "finish_kernels.cuh"
 #include "sort_policy.h"
 #include "tile_rank.cuh"
 
@@ -56,8 +57,8 @@ __device__ __noinline__ void write_pass_plan(uint32_t* plan, int num_passes, int
 // this CTA's shared counts (sh[pass * 256 + digit]) to the global ones, and the last CTA
 // to finish writes each pass's exclusive prefix (portion 0's digit bases) and, when asked,
 // the pass plan (the PLAN_* words: which passes skip, which buffers the others use).
-template <int TPB>
-__device__ __forceinline__ void histogram_finish(const HistogramParams& p, const uint32_t* sh)
+template <int TPB, class Route>
+__device__ __forceinline__ void histogram_finish(const HistogramParams& p, const uint32_t* sh, Route&& route)
 {
   constexpr int R = RADIX_DIGITS;
   __shared__ uint32_t last_flag;
@@ -115,37 +116,38 @@ __device__ __forceinline__ void histogram_finish(const HistogramParams& p, const
       }
     }
     unsigned long long run = x - s;
+    bool all_one_digit     = false;
     unsigned long long* out = p.bins + (size_t) warp * p.num_portions * R;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
     {
       out[lane * 8 + j] = run;
       run += c[j];
+      all_one_digit |= c[j] == p.num_items;
+    }
+    // a pass is skippable when one digit holds every key
+    if (__any_sync(0xffffffffu, all_one_digit) && lane == 0)
+    {
+      atomicOr(&trivial_mask, 1u << warp);
     }
   }
   if (p.plan == nullptr)
   {
     return;
   }
-  // a pass is skippable when one digit holds every key (counts re-read: fewer live registers)
-  if (warp < p.num_passes)
-  {
-    bool all_one_digit = false;
-#pragma unroll 1
-    for (int j = 0; j < 8; ++j)
-    {
-      all_one_digit |= __ldcg(&p.ctrl->counts[warp * R + lane * 8 + j]) == p.num_items;
-    }
-    if (__any_sync(0xffffffffu, all_one_digit) && lane == 0)
-    {
-      atomicOr(&trivial_mask, 1u << warp);
-    }
-  }
   __syncthreads();
   if (tid == 0)
   {
-    write_pass_plan(p.plan, p.num_passes, p.plan_mode, trivial_mask);
+    write_pass_plan(p.plan, p.num_passes, p.plan_mode, trivial_mask | route(trivial_mask));
   }
+}
+
+template <int TPB>
+__device__ __forceinline__ void histogram_finish(const HistogramParams& p, const uint32_t* sh)
+{
+  histogram_finish<TPB>(p, sh, [](uint32_t) {
+    return 0u;
+  });
 }
 
 // Calls fn(key) once for every key of keys[0, n), spread over the grid: a scalar head up
@@ -311,35 +313,49 @@ __device__ __forceinline__ void histogram_lanes_fold(unsigned char* table, uint3
   constexpr int R      = RADIX_DIGITS;
   constexpr bool PACKED = NP > 4;
   constexpr int ROWS   = PACKED ? (NP + 1) / 2 : NP; // word rows: pass pairs, or passes
+  constexpr int AHEAD  = 8; // rows read and summed together: their latencies overlap
   const int warp       = threadIdx.x >> 5;
   const int lane       = threadIdx.x & 31;
-  for (int r = warp; r < ROWS * R; r += TPB / 32)
+  static_assert(R % AHEAD == 0, "whole groups of rows");
+  for (int r0 = warp * AHEAD; r0 < ROWS * R; r0 += TPB / 32 * AHEAD)
   {
-    const int q          = r >> 8; // pass (pair, when packed)
-    const int d          = r & (R - 1);
-    const uint32_t base  = (uint32_t(q >> 1) << 16) | (uint32_t(d) << 8) | (uint32_t(q & 1) * 128u);
-    uint32_t* word       = reinterpret_cast<uint32_t*>(table + base + 4u * uint32_t(lane));
-    const uint32_t x     = *word;
-    *word                = 0u;
-    if constexpr (PACKED)
+    const int q          = r0 >> 8; // pass (pair, when packed)
+    const int d0         = r0 & (R - 1);
+    const uint32_t base  = (uint32_t(q >> 1) << 16) | (uint32_t(d0) << 8) | (uint32_t(q & 1) * 128u);
+    unsigned char* row   = table + base + 4u * uint32_t(lane);
+    uint32_t x[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
     {
-      const uint32_t lo = __reduce_add_sync(0xffffffffu, x & 0xffffu);
-      const uint32_t hi = __reduce_add_sync(0xffffffffu, x >> 16);
-      if (lane == 0)
+      uint32_t* word = reinterpret_cast<uint32_t*>(row + 256 * j);
+      x[j]           = *word;
+      *word          = 0u;
+    }
+    uint32_t lo = 0, hi = 0; // lane j: row r0 + j
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+    {
+      const uint32_t l = __reduce_add_sync(0xffffffffu, PACKED ? x[j] & 0xffffu : x[j]);
+      lo               = lane == j ? l : lo;
+      if constexpr (PACKED)
       {
-        totals[(2 * q) * R + d] += lo;
-        if (2 * q + 1 < NP)
-        {
-          totals[(2 * q + 1) * R + d] += hi;
-        }
+        const uint32_t h = __reduce_add_sync(0xffffffffu, x[j] >> 16);
+        hi               = lane == j ? h : hi;
       }
     }
-    else
+    if (lane < AHEAD)
     {
-      const uint32_t total = __reduce_add_sync(0xffffffffu, x);
-      if (lane == 0)
+      if constexpr (PACKED)
       {
-        totals[q * R + d] += total;
+        totals[(2 * q) * R + d0 + lane] += lo;
+        if (2 * q + 1 < NP)
+        {
+          totals[(2 * q + 1) * R + d0 + lane] += hi;
+        }
+      }
+      else
+      {
+        totals[q * R + d0 + lane] += lo;
       }
     }
   }
@@ -385,7 +401,7 @@ histogram_lanes_count(const HistogramParams& p, unsigned char* table, uint32_t t
     }
   }
   const uint4* vkeys              = reinterpret_cast<const uint4*>(keys + head);
-  const unsigned long long stride = (unsigned long long) gridDim.x * TPB;
+  const unsigned long long stride = (unsigned long long) (p.hist_ctas > 0 ? uint32_t(p.hist_ctas) : gridDim.x) * TPB;
   unsigned long long v            = blockIdx.x * (unsigned long long) TPB + tid;
   auto count_vec                  = [&](const uint4& w) {
     U k[VEC];
@@ -472,6 +488,15 @@ __device__ __forceinline__ void histogram_lanes_body(const HistogramParams& p)
   const int lane = tid & 31;
   const int P    = p.num_passes;
   const uint32_t table_bytes = uint32_t(histogram_table_bytes(P));
+  if constexpr (KB >= 4)
+  {
+    // the last CTAs sample the keys' top digits, one level each, before they count (or, for
+    // inputs that leave SMs idle, instead of counting)
+    if (p.finish != nullptr && blockIdx.x + uint32_t(p.sample_levels) >= gridDim.x)
+    {
+      finish_sample<KB, FP, TPB>(p, table, int(gridDim.x - blockIdx.x));
+    }
+  }
   for (uint32_t i = uint32_t(tid) * 16u; i < table_bytes; i += uint32_t(TPB) * 16u)
   {
     *reinterpret_cast<uint4*>(table + i) = make_uint4(0u, 0u, 0u, 0u);
@@ -494,7 +519,11 @@ __device__ __forceinline__ void histogram_lanes_body(const HistogramParams& p)
 
   // the pass count is a compile-time constant of the counting loop: a whole key, or a window;
   // the loop leaves the CTA's counts of (pass, digit) in sh
-  if (p.begin_bit == 0 && p.end_bit == 8 * KB)
+  if (p.hist_ctas > 0 && blockIdx.x >= uint32_t(p.hist_ctas))
+  {
+    // a CTA that only samples
+  }
+  else if (p.begin_bit == 0 && p.end_bit == 8 * KB)
   {
     histogram_lanes_count<KB, FP, TPB, KB, false>(p, table, table_base, col, sh);
   }
@@ -512,7 +541,16 @@ __device__ __forceinline__ void histogram_lanes_body(const HistogramParams& p)
       default: if constexpr (KB >= 8) { histogram_lanes_count<KB, FP, TPB, 8, true>(p, table, table_base, col, sh); } break;
     }
   }
-  histogram_finish<TPB>(p, sh);
+  if constexpr (KB >= 4)
+  {
+    histogram_finish<TPB>(p, sh, [&](uint32_t trivial_mask) {
+      return p.finish != nullptr ? finish_route<KB>(p, trivial_mask) : 0u;
+    });
+  }
+  else
+  {
+    histogram_finish<TPB>(p, sh);
+  }
 }
 
 // ---------------------------------------------------------------------------------------

@@ -10,6 +10,7 @@
 #include "radix_plan.h"
 
 #include <algorithm>
+#include <cmath>
 
 #include "abi_common.h"
 #include "sort_policy.h"
@@ -33,6 +34,7 @@ RadixPolicy make_radix_policy(int key_bytes, int value_bytes, int key_kind)
   p.persistent_items  = persistent_items(key_bytes, value_bytes);
   p.persistent_smem   = persistent_smem_bytes(key_bytes, value_bytes);
   p.single_tile_smem  = single_tile_smem_bytes(key_bytes);
+  p.finish            = finish_supported(key_bytes, value_bytes) ? 1 : 0;
   return p;
 }
 
@@ -48,6 +50,11 @@ RadixKernelNames radix_kernel_names(int kb, int vb, int kind, bool descending)
   n.onesweep_first = (vb == 0 && kind != KIND_FLOAT) ? "gb300_onesweep_first_" + kv : n.onesweep;
   // descending float sorts: CUB's single tile folds -0.0 into +0.0 before ordering (FP_BLOCK_DESC)
   n.single_tile = "gb300_single_tile_" + (kind == KIND_FLOAT && descending ? kv + "d" : kv);
+  if (finish_supported(kb, vb))
+  {
+    n.finish      = "gb300_finish_" + kv;
+    n.finish_tail = "gb300_finish_tail_" + kv;
+  }
   return n;
 }
 
@@ -73,15 +80,36 @@ plan_radix_temp(const RadixPolicy& pol, uint64_t n, int begin_bit, int end_bit, 
                                                uint64_t(pol.onesweep_tpb) * pol.onesweep_items);
   const uint64_t lookback_rows = ceil_div(n, min_tile) + t.num_portions;
 
+  // Partition and finish: whole keys, one portion (its indices have 32 bits), enough items.
+  t.finish = pol.finish == 1 && begin_bit == 0 && end_bit == 8 * pol.key_bytes && n >= finish_min_items(pol.key_bytes)
+          && t.num_portions == 1;
+
   size_t off     = 0;
   t.ctrl_off     = off;
   t.ctrl_bytes   = align_up(sizeof(SortControl) + 4 * size_t(t.num_passes) * t.num_portions, 256);
+  if (t.finish)
+  {
+    t.finish_ctrl_off = t.ctrl_off + t.ctrl_bytes;
+    t.ctrl_bytes += align_up(sizeof(FinishControl), 256);
+  }
   off += t.ctrl_bytes;
   t.bins_off = off;
   off += align_up(8 * size_t(t.num_passes) * t.num_portions * RADIX_DIGITS, 256);
   t.lookback_off   = off;
   t.lookback_words = size_t(lookback_rows) * RADIX_DIGITS;
   off += align_up(2 * 4 * t.lookback_words, 256);
+  if (t.finish)
+  {
+    t.finish_pieces = ceil_div(n, uint64_t(finish_cap(pol.key_bytes, pol.value_bytes, false)) / FINISH_SMALLEST_PIECE);
+    t.rest_off      = off;
+    off += align_up(sizeof(FinishRange) * t.finish_pieces, 256);
+    t.large_off = off;
+    off += align_up(sizeof(FinishRange) * t.finish_pieces, 256);
+    t.offsets_off = off;
+    off += align_up(4 * t.finish_pieces, 256);
+    t.table_off = off;
+    off += 4 * size_t(RADIX_DIGITS) * FINISH_MAX_CTAS;
+  }
   t.keys_tmp_off = off;
   if (need_tmp)
   {
@@ -239,6 +267,9 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
                       reinterpret_cast<uint32_t*>(base + t.lookback_off) + t.lookback_words};
   void* keys_tmp   = base + t.keys_tmp_off;
   void* values_tmp = base + t.values_tmp_off;
+  // buffers that are not 16-byte aligned take every pass (the finish bulk-copies its pieces)
+  const bool finish = t.finish && persistent && ks.finish != nullptr;
+  auto* fctrl       = reinterpret_cast<FinishControl*>(base + t.finish_ctrl_off);
 
   // 1. zero the control block (histogram counters, tile counters, status)
   {
@@ -269,7 +300,34 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
     p.plan_mode = c.overwrite ? PLAN_MODE_DOUBLE : PLAN_MODE_SEPARATE;
     // one lane-column CTA per SM (fewer for small inputs: four 16-byte loads per thread)
     const uint64_t want = ceil_div(n, uint64_t(HISTOGRAM_LANES_TPB) * (16 / kb) * 4);
-    const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(sm_count()))));
+    unsigned grid       = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(sm_count()))));
+    p.hist_ctas         = int(grid);
+    if (finish)
+    {
+      // one CTA per level of digits samples the keys, on idle SMs where there are any
+      p.finish        = fctrl;
+      p.sample_levels = kb;
+      p.sample_items  = finish_sample_items(n);
+      p.finish_cap    = uint32_t(finish_cap(kb, vb, false));
+      p.finish_cost   = finish_cost(kb, vb);
+      // sampled keys of one bucket that no bucket of p.finish_cap items would plausibly give
+      const double mean = double(p.finish_cap) * p.sample_items / double(n);
+      auto heavy        = [](double m) {
+        return uint32_t(2.0 + 1.3 * m + 4.0 * std::sqrt(m) + 0.5);
+      };
+      p.sample_heavy       = heavy(mean);
+      p.sample_heavy_first = heavy(mean * HISTOGRAM_LANES_TPB / p.sample_items);
+      // The sampling CTAs count keys too only where that takes longer than the sample (keys of
+      // more than 2^30 bytes); below, the other CTAs are done before they would be.
+      const unsigned sms    = unsigned(sm_count());
+      const unsigned levels = unsigned(kb);
+      if (n * uint64_t(kb) <= (1ull << 30) && grid + levels > sms)
+      {
+        grid = sms - levels;
+      }
+      p.hist_ctas = int(grid);
+      grid        = std::min(grid + levels, sms);
+    }
     launch("histogram", ks.histogram, grid, unsigned(HISTOGRAM_LANES_TPB), histogram_table_bytes(passes), c.stream, p);
   }
   // 3. one onesweep launch per (pass, portion)
@@ -296,6 +354,7 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
     }
   }
   const uint64_t tiles_per_portion = t.portion_items / t.tile_items;
+  uint32_t* const status           = c.status_word != nullptr ? c.status_word : &ctrl->status;
   // buffer tables of the pass plan (PLAN_MODE_DOUBLE: {current, alternate};
   // PLAN_MODE_SEPARATE: {input, output, temporary})
   const void* key_bufs[3]   = {c.keys[0], c.keys[1], c.overwrite ? nullptr : keys_tmp};
@@ -323,7 +382,7 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
       op.tile_counter  = tile_ctrs + (size_t(p) * t.num_portions + q);
       op.bins          = bins + (size_t(p) * t.num_portions + q) * RADIX_DIGITS;
       op.bins_next     = (q + 1 < t.num_portions) ? bins + (size_t(p) * t.num_portions + q + 1) * RADIX_DIGITS : nullptr;
-      op.status        = c.status_word != nullptr ? c.status_word : &ctrl->status;
+      op.status        = status;
       op.codec         = codec;
       op.current_bit   = bit;
       op.num_bits      = std::min(RADIX_BITS, c.end_bit - bit);
@@ -352,6 +411,35 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
                op);
       }
     }
+  }
+  // 4. partition and finish, when the histogram's sample chose it: the result of the passes that
+  // ran is in the buffer every pass running would leave it in, and is finished there
+  if (finish)
+  {
+    const int result = passes & 1; // with overwrite: the buffer every pass running ends in
+    FinishParams fp{};
+    fp.keys        = c.overwrite ? c.keys[result] : c.keys[1];
+    fp.values      = !has_vals ? nullptr : c.overwrite ? c.values[result] : c.values[1];
+    fp.free_keys   = c.overwrite ? c.keys[result ^ 1] : keys_tmp;
+    fp.free_values = !has_vals ? nullptr : c.overwrite ? c.values[result ^ 1] : values_tmp;
+    fp.num_items   = uint32_t(n);
+    fp.ctrl        = fctrl;
+    fp.rest        = reinterpret_cast<FinishRange*>(base + t.rest_off);
+    fp.large       = reinterpret_cast<FinishRange*>(base + t.large_off);
+    fp.offsets     = reinterpret_cast<uint32_t*>(base + t.offsets_off);
+    fp.table       = reinterpret_cast<uint32_t*>(base + t.table_off);
+    fp.status      = status;
+    fp.codec       = codec;
+    fp.gate        = c.gate;
+    const uint64_t sms  = uint64_t(sm_count());
+    const unsigned tpb  = unsigned(finish_tpb(kb, vb, false)) + 32;
+    const size_t smem   = finish_smem_bytes(kb, vb, false);
+    const uint64_t most = sms * occupancy(ks.finish, int(tpb), smem);
+    launch("finish", ks.finish, unsigned(std::min<uint64_t>(t.finish_pieces, most)), tpb, smem, c.stream, fp);
+    const unsigned ttpb = unsigned(finish_tpb(kb, vb, true)) + 32;
+    const size_t tsmem  = finish_smem_bytes(kb, vb, true);
+    launch_cooperative("finish_tail", ks.finish_tail, unsigned(std::min<uint64_t>(sms, FINISH_MAX_CTAS)), ttpb, tsmem,
+                       c.stream, fp);
   }
   *selector = passes & 1;
 }

@@ -29,7 +29,8 @@ struct RadixPolicy
   int32_t persistent_tpb;
   int32_t persistent_items;
   int32_t gather_value_bytes; // > 0: the caller's values have this width, sorted as 32-bit indices
-  int32_t reserved[4];
+  int32_t finish; // 1: the image holds the partition-and-finish kernels (blobs of older builds: 0)
+  int32_t reserved[3];
   uint64_t onesweep_smem;
   uint64_t single_tile_smem;
   uint64_t persistent_smem;
@@ -45,12 +46,15 @@ struct RadixKernels
   CUkernel onesweep_first; // its order-free variant for pass 0 of integer keys-only sorts (may be == onesweep)
   CUkernel onesweep_dyn;   // CTA-per-tile pass kernel for buffers that are not 16-byte aligned
   CUkernel single_tile;
+  CUkernel finish; // partition and finish (finish_kernels.cuh); unused unless RadixPolicy::finish
+  CUkernel finish_tail;
 };
 
 // Kernel names of one (key width, value width, key kind) in the radix image.
 struct RadixKernelNames
 {
   std::string init, histogram, onesweep, onesweep_first, onesweep_dyn, single_tile;
+  std::string finish, finish_tail; // empty where the finish does not carry the types
 };
 RadixKernelNames radix_kernel_names(int key_bytes, int value_bytes, int key_kind, bool descending);
 
@@ -83,6 +87,10 @@ struct RadixTempPlan
   size_t bins_off;
   size_t lookback_off, lookback_words; // two buffers of lookback_words each
   size_t keys_tmp_off, values_tmp_off;
+  bool finish;                // the sizes qualify for the partition-and-finish route
+  uint64_t finish_pieces;     // most pieces of that route
+  size_t finish_ctrl_off;     // FinishControl, in the control block
+  size_t rest_off, large_off, offsets_off, table_off;
   size_t total_bytes;
 };
 

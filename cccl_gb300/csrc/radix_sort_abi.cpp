@@ -163,8 +163,9 @@ try
   r.runtime_policy       = pol;
   r.runtime_policy_size  = sizeof(RadixPolicy);
   r.single_tile_kernel_lowered_name            = dup_cstr(st);
-  r.upsweep_kernel_lowered_name                = dup_cstr(his);
-  r.alt_upsweep_kernel_lowered_name            = dup_cstr(his);
+  const bool fin = pol->finish == 1;
+  r.upsweep_kernel_lowered_name                = dup_cstr(fin ? names.finish : his);
+  r.alt_upsweep_kernel_lowered_name            = dup_cstr(fin ? names.finish_tail : his);
   r.scan_bins_kernel_lowered_name              = dup_cstr(his);
   r.downsweep_kernel_lowered_name              = dup_cstr(dyn);
   r.alt_downsweep_kernel_lowered_name          = dup_cstr(first);
@@ -349,7 +350,9 @@ CCCL_C_API CUresult cccl_device_radix_sort(
                     build.onesweep_kernel,
                     build.alt_downsweep_kernel,
                     build.downsweep_kernel,
-                    build.single_tile_kernel};
+                    build.single_tile_kernel,
+                    build.upsweep_kernel,
+                    build.alt_upsweep_kernel};
     RadixCall call{};
     call.keys[0]          = d_keys_in.state;
     call.keys[1]          = d_keys_out.state;

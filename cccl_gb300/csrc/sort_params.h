@@ -104,6 +104,26 @@ struct InitParams
   KernelGate gate;
 };
 
+// Partition-and-finish route of a plain sort (finish_kernels.cuh), in the control block;
+// zeroed with it, written by the histogram kernel.
+struct FinishControl
+{
+  uint32_t route;        // 0: every digit pass runs; 1: top digits, then the finish
+  uint32_t piece_items;  // the finish cuts the array at bucket starts about this far apart
+  uint32_t num_pieces;
+  uint32_t prefix_shift; // low key bits the partition did not sort by
+  uint32_t ticket;       // next piece
+  uint32_t barrier;      // grid-wide barrier of the rest kernel
+  uint32_t large_pieces; // pieces listed in FinishParams::large
+  uint32_t large_ticket;
+  uint32_t search_step;    // a power of 8
+  uint32_t pad;
+  unsigned long long rest_items;
+  // sample of the keys' top 1, 2, .. digits (finish_sample)
+  unsigned long long light[MAX_PASSES];
+  uint32_t heavy[MAX_PASSES];
+};
+
 struct HistogramParams
 {
   const void* keys;
@@ -120,7 +140,39 @@ struct HistogramParams
   KernelGate gate;
   uint32_t* plan;             // [num_passes] pass plan words to write, or null (no skipping)
   int plan_mode;              // PLAN_MODE_*
-  int pad0;
+  int hist_ctas;              // CTAs that count keys (0: all); the last sample_levels CTAs sample
+  FinishControl* finish;      // null: every digit pass runs
+  int sample_levels;
+  uint32_t sample_items;      // keys sampled: 2^12 or 2^13
+  uint32_t sample_heavy;      // sampled keys of one prefix that make its bucket too large
+  uint32_t sample_heavy_first; // the same for the first 2^10 sampled keys alone
+  uint32_t finish_cap;        // largest piece the finish's first launch takes
+  float finish_cost;          // time of the finish, in digit passes
+};
+
+// Pieces of the partitioned array (finish_kernels.cuh).
+struct FinishRange
+{
+  uint32_t begin;
+  uint32_t items;
+};
+
+struct FinishParams
+{
+  void* keys; // the partitioned raw keys, sorted in place
+  void* values;
+  void* free_keys; // another buffer of the array's size
+  void* free_values;
+  uint32_t num_items;
+  uint32_t pad0;
+  FinishControl* ctrl;
+  FinishRange* rest;  // [num_pieces]: what finish_tail sorts as one sequence (items 0: nothing)
+  FinishRange* large; // [num_pieces]: pieces for the general form
+  uint32_t* offsets;  // [num_pieces]
+  uint32_t* table;    // [FINISH_MAX_CTAS][256]
+  uint32_t* status;
+  KeyCodec codec;
+  KernelGate gate;
 };
 
 struct OnesweepParams

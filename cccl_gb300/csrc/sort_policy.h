@@ -8,6 +8,7 @@
 // dynamic shared memory, so the staging tile is sized by registers, not by the 48 KB cap.
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 
 #include "sort_params.h"
@@ -203,6 +204,157 @@ GB300_HD inline void plan_pass_words(uint32_t* plan, int num_passes, int plan_mo
     }
     plan[q] = w;
   }
+}
+
+// ---- partition and finish (finish_kernels.cuh) ----
+constexpr int FINISH_BIN_MAX        = 64;      // keys of a bin that the common form of the finish takes
+constexpr int FINISH_KNOTS          = 32;      // stretches of a large piece's bins
+constexpr int FINISH_SMALLEST_PIECE = 2;       // piece_items is at least CAP / 2
+constexpr int FINISH_REST_ITEMS     = 4;
+constexpr int FINISH_MAX_CTAS       = 304;     // of finish_tail
+
+GB300_HD constexpr bool finish_supported(int kb, int vb)
+{
+  return (kb == 4 || kb == 8) && (vb == 0 || vb == 4 || vb == 8);
+}
+// Sorting threads and items per thread of the finish (one more warp fetches): two CTAs per SM,
+// as large as shared memory lets them be. The buckets of 2^28 uniform keys split 2^16 ways hold
+// 4096 +- 5 x 64 keys, and a piece must take one whole. Twelve items: four-word groups at a
+// stride of 12 words are free of bank conflicts. Measured, ps per item (2^28 u64 + u32, 2^28 u32,
+// 2^26 f64 + i64): 480 x 12 6.0 / 4.4 / -, 736 x 8 6.8 / 4.9 / -, 608 x 8 6.0 / 4.4 / 6.6,
+// 768 x 8 with one CTA per SM - / - / 9.9, 416 x 12 - / - / 6.5.
+// Its second launch (large) takes pieces of up to twice the size, one CTA per SM: the densest
+// buckets of a normal distribution hold twice as many keys as the mean one.
+constexpr int FINISH_ITEMS = 12;
+GB300_HD constexpr int finish_tpb(int kb, int vb, bool large)
+{
+  return large ? (kb + vb == 16 ? 864 : 960) : (kb + vb == 16 ? 416 : 480);
+}
+GB300_HD constexpr int finish_minb(bool large)
+{
+  return large ? 1 : 2;
+}
+// Equal parts of a piece's key range, 8 per sorting thread (16: 6.3 / 4.9 ps per item).
+GB300_HD constexpr int finish_bins(int kb, int vb, bool large)
+{
+  return finish_tpb(kb, vb, large) * 8;
+}
+GB300_HD constexpr int finish_cap(int kb, int vb, bool large)
+{
+  return finish_tpb(kb, vb, large) * FINISH_ITEMS;
+}
+GB300_HD constexpr size_t finish_smem_bytes(int kb, int vb, bool large)
+{
+  const size_t cap = size_t(finish_cap(kb, vb, large));
+  return round16(kb * cap) + 16 + (vb > 0 ? round16(vb * cap) + 16 : 0) + size_t(2) * finish_bins(kb, vb, large)
+       + round16(4 * cap) + (large ? size_t(24) * FINISH_KNOTS : 0) + 512;
+}
+// Smallest sort that takes the sample and, if it promises enough, the partition-and-finish route:
+// below, the sample and two launches (17 us at 2^22 items) weigh too much where it is not taken.
+// Four-byte keys gain less (2 passes of 4).
+GB300_HD constexpr unsigned long long finish_min_items(int kb)
+{
+  return kb == 8 ? 1ull << 22 : 1ull << 26;
+}
+// Time of the finish and its bounds in digit passes of the same items (measured at 2^28 items: u64 +
+// u32 1.8 ms against 1.66, u32 1.31 against 0.93).
+GB300_HD constexpr float finish_cost(int kb, int vb)
+{
+  return (void) vb, kb == 8 ? 1.1f : 1.4f;
+}
+// Sampled keys: more for larger inputs, whose buckets hold a smaller share of the keys.
+GB300_HD constexpr unsigned finish_sample_items(unsigned long long n)
+{
+  return n >= (1ull << 24) ? 8192u : 4096u; // a 64 KB table and 8 bytes a key: 128 KB
+}
+
+// Top digits to partition by (0: run every digit pass). `trivial_mask`: passes whose digit is
+// constant; light[l] and heavy[l]: what the sample of S keys found for the top l + 1 digits
+// (finish_sample; for whole keys: groups of two and three, and all small groups). The mean number of other keys in the bucket of a sampled key is n / S times
+// the mean number of other sampled keys in it. A candidate
+//   * must leave buckets of at most 0.85 of the finish's capacity in that mean (up to 2.4 times
+//     the mean then fits its second launch);
+//   * must not crowd the finish's bins (FINISH_BIN_MAX): they split a piece 3328 or 3840 ways, so
+//     a bucket that fills it 11.8 bits further down, a smaller one fewer bits. The mean number of
+//     other keys there, read between the levels of the sample, may be 3 at most (a smooth density
+//     leaves about one), a digit further down there must be far fewer pairs, here and at the levels
+//     above (keys that cluster at every scale, such as ANDs of random words, show no other
+//     sign), and the mean key may have 6 equals at most;
+//   * must cost less: the partition passes, the finish and, for the share of the keys in large
+//     groups, the rest kernel's passes at half speed, half a pass less than all passes;
+//   * may need half of the passes at most: where it takes more digits to part the keys they
+//     cluster at every scale, and the pieces would too.
+GB300_HD inline int finish_choose(int kb, uint32_t trivial_mask, const unsigned long long* light, const uint32_t* heavy,
+                                  unsigned long long n, uint32_t samples, uint32_t cap, float cost, int plan_mode,
+                                  uint32_t* piece_items)
+{
+  int total = 0;
+  for (int q = 0; q < kb; ++q)
+  {
+    total += (trivial_mask >> q) & 1u ? 0 : 1;
+  }
+  const float scale = float(n) / float(samples) / float(samples);
+  // Mean number of other keys at every level. `sure`: what is left of it 1.5 standard deviations
+  // of the pairs found below; no pair: fewer than about a third of one, and no more than a
+  // smooth density gives from the level above.
+  // The groups of four and more equal keys do not count (zeros: one crowded piece or bucket).
+  const float repeated = float(heavy[kb - 1]) - float(light[kb - 1]);
+  float others[8], sure[8];
+  for (int l = 0; l < kb; ++l)
+  {
+    const float found = l < kb - 1 ? (float(light[l]) > repeated ? float(light[l]) - repeated : 0.0f) : float(light[l]);
+    others[l]         = found * scale;
+    const float pairs = 0.5f * found;
+    sure[l]           = 2.0f * (pairs - 1.5f * sqrtf(pairs)) * scale;
+    if (pairs <= 2.25f)
+    {
+      const float smooth = l > 0 ? sure[l - 1] / 128.0f : 0.6f * scale;
+      sure[l]            = smooth < 0.6f * scale ? smooth : 0.6f * scale;
+    }
+    sure[l] = sure[l] > 1e-20f ? sure[l] : 1e-20f;
+  }
+  if (others[kb - 1] > 6.0f)
+  {
+    return 0;
+  }
+  int passes = 0;
+  for (int digits = 1; digits < kb; ++digits)
+  {
+    // keys that cluster at every scale: a smooth density has 256 times fewer pairs a digit down
+    // (pairs of equal keys aside)
+    const float pairs = 0.5f * float(light[digits - 1]);
+    const float below = 0.5f * (float(light[digits]) - float(heavy[kb - 1]));
+    if (pairs >= 16.0f && heavy[digits - 1] < samples / 64u && digits < kb - 1 && below > pairs / 128.0f + 3.0f)
+    {
+      return 0;
+    }
+    passes += (trivial_mask >> (kb - digits)) & 1u ? 0 : 1;
+    const int run      = plan_mode == PLAN_MODE_DOUBLE && (passes & 1) ? passes + 1 : passes;
+    const float large  = float(heavy[digits - 1]) / float(samples);
+    const float bucket = 1.0f + others[digits - 1];
+    if (passes == 0 || 2 * run > total || bucket > 0.85f * float(cap)
+        || float(run) + cost + 2.0f * float(kb) * large > float(total) - 0.5f)
+    {
+      continue;
+    }
+    // pieces about this far apart, so that most hold whole buckets up to the capacity
+    float piece = float(cap) - 1.25f * bucket;
+    piece       = piece < float(cap) / FINISH_SMALLEST_PIECE ? float(cap) / FINISH_SMALLEST_PIECE : piece;
+    piece       = piece > 0.875f * float(cap) ? 0.875f * float(cap) : piece;
+    // bits below the bucket that the bins resolve, as a place between the sample's levels
+    const float share = piece / bucket > 1.0f ? piece / bucket : 1.0f;
+    float level       = float(digits) + (11.8f - log2f(share)) / 8.0f;
+    level             = level < float(digits) ? float(digits) : level > float(kb) ? float(kb) : level;
+    const int upper   = level >= float(kb) ? kb - 1 : int(level);
+    const float bin   = sure[upper - 1] * exp2f((level - float(upper)) * log2f(sure[upper] / sure[upper - 1]));
+    if (bin > 3.0f)
+    {
+      continue;
+    }
+    *piece_items = uint32_t(piece);
+    return digits;
+  }
+  return 0;
 }
 
 GB300_HD constexpr int single_tile_capacity()

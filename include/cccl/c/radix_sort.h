@@ -20,8 +20,11 @@
  *      single_tile_kernel            whole sort in one CTA for small inputs
  *      alt_downsweep_kernel          first-pass variant for full-width integer keys-only
  *                                    sorts (order inside a digit bucket is free there)
- *      upsweep/scan_bins/alt_upsweep: CUB's multi-pass kernels are never used on
- *      sm_90+; these members alias the histogram kernel so they are non-null.
+ *      upsweep_kernel, alt_upsweep_kernel  whole 4- and 8-byte keys with values of 0, 4 or 8
+ *                                    bytes: the two kernels that finish a sort partitioned by its
+ *                                    top digits; else the histogram kernel
+ *      scan_bins_kernel              the histogram kernel (CUB's multi-pass kernels are never
+ *                                    used on sm_90+), so that the member is non-null
  *  - runtime_policy: the tile configuration chosen for the key/value types.
  */
 #pragma once

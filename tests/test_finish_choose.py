@@ -1,0 +1,20 @@
+"""The plain sort's choice between all digit passes and the top ones (finish_choose in
+cccl_gb300/csrc/sort_policy.h, the code the histogram kernel runs) and the finish kernels'
+shapes, compiled with g++ (tests/host/finish_choose_check.cpp)."""
+
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_digits_chosen(tmp_path):
+    exe = tmp_path / "finish_choose_check"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-I", str(ROOT / "cccl_gb300" / "csrc"),
+                    str(ROOT / "tests" / "host" / "finish_choose_check.cpp"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
