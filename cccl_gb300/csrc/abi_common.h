@@ -209,6 +209,44 @@ inline void launch(
   notify_launch(role, 1, stream);
 }
 
+// Launch that may start while the grid before it in the stream ends (chained): the kernel waits for
+// that grid itself (wait_for_previous_grid), so its launch and its CTAs' start are not added to the
+// stream's time. A chain of short kernels takes 1.6 us a launch instead of 4.2 (GB300).
+template <class Params>
+inline void launch_after(
+  const char* role, CUkernel kernel, unsigned grid, unsigned block, size_t smem, CUstream stream, const Params& p, bool chained)
+{
+  if (!chained)
+  {
+    launch(role, kernel, grid, block, smem, stream, p);
+    return;
+  }
+  CUfunction f = function_of(kernel);
+  if (smem > 47 * 1024)
+  {
+    check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
+          "cuFuncSetAttribute(max dynamic shared memory)");
+  }
+  CUlaunchAttribute attr{};
+  attr.id                                         = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  attr.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig config{};
+  config.gridDimX       = grid;
+  config.gridDimY       = 1;
+  config.gridDimZ       = 1;
+  config.blockDimX      = block;
+  config.blockDimY      = 1;
+  config.blockDimZ      = 1;
+  config.sharedMemBytes = unsigned(smem);
+  config.hStream        = stream;
+  config.attrs          = &attr;
+  config.numAttrs       = 1;
+  void* args[]          = {const_cast<Params*>(&p)};
+  notify_launch(role, 0, stream);
+  check(cuLaunchKernelEx(&config, f, args, nullptr), "cuLaunchKernelEx");
+  notify_launch(role, 1, stream);
+}
+
 // Cooperative launch: every CTA of the grid is resident at once (the persistent kernels
 // wait on each other's tiles, so co-residency is required for forward progress).
 template <class Params>

@@ -972,6 +972,11 @@ __device__ __forceinline__ void finish_body(const FinishParams& p)
           asm volatile("bar.sync 2, %0;" ::"n"(TPB + 32) : "memory"); // the previous piece is written out
           fence_proxy_async_smem();
           failed = *reinterpret_cast<volatile uint32_t*>(word + 2) != 0u;
+          if (LARGE && lane == 0)
+          {
+            __threadfence();
+            atomicAdd(&p.ctrl->large_done, 1u);
+          }
         }
         if (items == 0u || failed)
         {
@@ -1097,19 +1102,17 @@ __device__ __forceinline__ void finish_body(const FinishParams& p)
 // order, so the sequence sorted as a whole is the pieces sorted one by one: its items are
 // gathered into one half of the free buffer, sorted there by LSD digit passes between the two
 // halves, and put back. When they are more than half of the array the whole array is sorted
-// instead, between its own buffer and the free one. It shares a cooperative launch with the large
-// pieces (finish_tail), with grid-wide barriers (every wait bounded): most sorts have neither,
+// instead, between its own buffer and the free one. It shares a launch with the large pieces
+// (finish_tail), in phases of work (finish_phase; every wait bounded): most sorts have neither,
 // and should pay one empty launch for both, not a pass sequence.
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ bool finish_grid_sync(uint32_t* counter, uint32_t ctas, uint32_t& target, uint32_t* status)
+// Waits (bounded) until *counter reaches `target`. Called by the whole CTA.
+__device__ __forceinline__ bool finish_wait_for(const uint32_t* counter, uint32_t target, uint32_t* status)
 {
   __shared__ uint32_t ok;
   __syncthreads();
-  target += ctas;
   if (threadIdx.x == 0)
   {
-    __threadfence();
-    atomicAdd(counter, 1u);
     const uint64_t start = global_timer_ns();
     bool arrived         = true;
     while (load_status(counter) < target)
@@ -1127,6 +1130,40 @@ __device__ __forceinline__ bool finish_grid_sync(uint32_t* counter, uint32_t cta
   }
   __syncthreads();
   return ok != 0u;
+}
+
+// One phase of work in `units` units: every CTA takes units (body(unit)) until none is left, then
+// waits for those that others took. Only units that a running CTA took are waited for, so CTAs
+// that have not started yet, or never do, hold nobody up.
+template <class Body>
+__device__ __forceinline__ bool
+finish_phase(FinishControl* ctrl, int& phase, uint32_t units, uint32_t* status, Body&& body)
+{
+  __shared__ uint32_t unit;
+  while (true)
+  {
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+      unit = atomicAdd(&ctrl->claimed[phase], 1u);
+    }
+    __syncthreads();
+    const uint32_t b = unit;
+    if (b >= units)
+    {
+      break;
+    }
+    body(b);
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+      __threadfence();
+      atomicAdd(&ctrl->done[phase], 1u);
+    }
+  }
+  const bool ok = finish_wait_for(&ctrl->done[phase], units, status);
+  ++phase;
+  return ok;
 }
 
 // Sum of v over the CTA, returned to every thread; scratch: TPB / 32 words.
@@ -1183,16 +1220,15 @@ __device__ __forceinline__ void finish_rest_body(const FinishParams& p)
   }
   __syncthreads();
   const int tid         = threadIdx.x;
-  const uint32_t b      = blockIdx.x;
   const uint32_t n      = p.num_items;
   const uint32_t pieces = __ldcg(&p.ctrl->num_pieces);
   const bool whole      = 2 * found + 64 > n;
   const uint32_t m      = whole ? n : uint32_t(found);
-  // few items take few CTAs: a barrier and the walk over the CTAs' digit counts cost less
-  const uint32_t G = min(gridDim.x, (m + TILE - 1) / TILE);
-  if (b >= G)
+  // The sequence in G shares. Few items make few: the walk over the shares' digit counts costs less.
+  const uint32_t G = min(min(gridDim.x, uint32_t(FINISH_MAX_CTAS)), (m + TILE - 1) / TILE);
+  if (whole && !finish_wait_for(&p.ctrl->large_done, __ldcg(&p.ctrl->large_pieces), p.status))
   {
-    return;
+    return; // the large pieces are part of the array: all of them have to be written
   }
   // the two buffers of the passes
   U* keys   = static_cast<U*>(p.keys);
@@ -1203,14 +1239,18 @@ __device__ __forceinline__ void finish_rest_body(const FinishParams& p)
   vbuf[0] = whole ? values : static_cast<V*>(p.free_values);
   kbuf[1] = static_cast<U*>(p.free_keys) + (whole ? 0u : (m + 15u) & ~15u);
   vbuf[1] = static_cast<V*>(p.free_values) + (whole ? 0u : (m + 15u) & ~15u);
-  uint32_t target = 0;
-  // this CTA's share of the sequence
   const uint32_t share = (m + G - 1) / G;
-  const uint32_t v0    = min(b * share, m);
-  const uint32_t v1    = min(v0 + share, m);
+  auto share_begin     = [&](uint32_t b) {
+    return min(b * share, m);
+  };
+  int phase_no = 0;
+  auto phase   = [&](auto&& body) {
+    return finish_phase(p.ctrl, phase_no, G, p.status, body);
+  };
 
-  // moves items between their places in the array and the sequence
-  auto transfer = [&](bool gather, int buffer) {
+  // moves a share's items between their places in the array and the sequence
+  auto transfer = [&](uint32_t b, bool gather, int buffer) {
+    const uint32_t v0 = share_begin(b), v1 = share_begin(b + 1u);
     uint32_t c = 0, first = 0, items = 0; // current piece: [first, first + items) of the sequence
     for (uint32_t v = v0 + tid; v < v1; v += TPB)
     {
@@ -1259,130 +1299,121 @@ __device__ __forceinline__ void finish_rest_body(const FinishParams& p)
 
   if (!whole)
   {
-    // offsets of the pieces in the sequence
+    // offsets of the pieces in the sequence: sums over stretches of pieces, then their prefixes
     const uint32_t per = (pieces + G - 1) / G;
-    const uint32_t c0  = min(b * per, pieces);
-    const uint32_t c1  = min(c0 + per, pieces);
-    uint32_t sum       = 0;
-    for (uint32_t c = c0 + tid; c < c1; c += TPB)
-    {
-      sum += __ldcg(&p.rest[c].items);
-    }
-    sum = finish_block_sum<TPB>(sum, scratch);
-    if (tid == 0)
-    {
-      p.table[b] = sum;
-    }
-    if (!finish_grid_sync(&p.ctrl->barrier, G, target, p.status))
-    {
-      return;
-    }
-    uint32_t before = 0;
-    for (uint32_t c = tid; c < b; c += TPB)
-    {
-      before += __ldcg(p.table + c);
-    }
-    before = finish_block_sum<TPB>(before, scratch);
-    for (uint32_t c = c0; c < c1; c += TPB)
-    {
-      const uint32_t mine = c + tid < c1 ? __ldcg(&p.rest[c + tid].items) : 0u;
-      uint32_t x          = mine;
+    const bool ok      = phase([&](uint32_t b) {
+      const uint32_t c0 = min(b * per, pieces), c1 = min(c0 + per, pieces);
+      uint32_t sum      = 0;
+      for (uint32_t c = c0 + tid; c < c1; c += TPB)
+      {
+        sum += __ldcg(&p.rest[c].items);
+      }
+      sum = finish_block_sum<TPB>(sum, scratch);
+      if (tid == 0)
+      {
+        p.table[b] = sum;
+      }
+    })
+    && phase([&](uint32_t b) {
+      const uint32_t c0 = min(b * per, pieces), c1 = min(c0 + per, pieces);
+      uint32_t before   = 0;
+      for (uint32_t c = tid; c < b; c += TPB)
+      {
+        before += __ldcg(p.table + c);
+      }
+      before = finish_block_sum<TPB>(before, scratch);
+      for (uint32_t c = c0; c < c1; c += TPB)
+      {
+        const uint32_t mine = c + tid < c1 ? __ldcg(&p.rest[c + tid].items) : 0u;
+        uint32_t x          = mine;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1)
-      {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if ((tid & 31) >= o)
+        for (int o = 1; o < 32; o <<= 1)
         {
-          x += y;
+          const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+          if ((tid & 31) >= o)
+          {
+            x += y;
+          }
         }
+        __syncthreads();
+        if ((tid & 31) == 31)
+        {
+          scratch[tid >> 5] = x;
+        }
+        __syncthreads();
+        uint32_t all = 0, warps_before = 0;
+        for (int w = 0; w < NW; ++w)
+        {
+          warps_before += w < (tid >> 5) ? scratch[w] : 0u;
+          all += scratch[w];
+        }
+        if (c + tid < c1)
+        {
+          p.offsets[c + tid] = before + warps_before + x - mine;
+        }
+        before += all;
       }
-      __syncthreads();
-      if ((tid & 31) == 31)
-      {
-        scratch[tid >> 5] = x;
-      }
-      __syncthreads();
-      uint32_t all = 0, warps_before = 0;
-      for (int w = 0; w < NW; ++w)
-      {
-        warps_before += w < (tid >> 5) ? scratch[w] : 0u;
-        all += scratch[w];
-      }
-      if (c + tid < c1)
-      {
-        p.offsets[c + tid] = before + warps_before + x - mine;
-      }
-      before += all;
-    }
-    if (!finish_grid_sync(&p.ctrl->barrier, G, target, p.status))
-    {
-      return;
-    }
-    transfer(true, 0);
-    if (!finish_grid_sync(&p.ctrl->barrier, G, target, p.status))
+    })
+    && phase([&](uint32_t b) {
+      transfer(b, true, 0);
+    });
+    if (!ok)
     {
       return;
     }
   }
 
   // digits in which two keys differ: the others need no pass
-  uint32_t vary = 0;
+  uint32_t* bits = p.table + size_t(FINISH_MAX_CTAS) * R; // [G][KB / 4][2] bits set, bits clear in a share's keys
+  if (!phase([&](uint32_t b) {
+        U ones = U(0), zeros = U(0);
+        const uint32_t v1 = share_begin(b + 1u);
+        for (uint32_t v = share_begin(b) + tid; v < v1; v += TPB)
+        {
+          const U t = digit_source<U, FP>(encode_key<U>(__ldcg(kbuf[0] + v), p.codec));
+          ones |= t;
+          zeros |= U(~t);
+        }
+        if (tid < 8)
+        {
+          dscratch[tid] = 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < KB / 4; ++j)
+        {
+          const uint32_t o = __reduce_or_sync(0xffffffffu, uint32_t((unsigned long long) ones >> (32 * j)));
+          const uint32_t z = __reduce_or_sync(0xffffffffu, uint32_t((unsigned long long) zeros >> (32 * j)));
+          if ((tid & 31) == 0)
+          {
+            atomicOr(&dscratch[2 * j], o);
+            atomicOr(&dscratch[2 * j + 1], z);
+          }
+        }
+        __syncthreads();
+        if (tid < KB / 2)
+        {
+          bits[b * (KB / 2) + tid] = dscratch[tid];
+        }
+      }))
   {
-    U ones = U(0), zeros = U(0);
-    for (uint32_t v = v0 + tid; v < v1; v += TPB)
-    {
-      const U t = digit_source<U, FP>(encode_key<U>(__ldcg(kbuf[0] + v), p.codec));
-      ones |= t;
-      zeros |= U(~t);
-    }
-    uint32_t digits1 = 0, digits0 = 0;
+    return;
+  }
+  uint32_t vary = 0;
 #pragma unroll
-    for (int j = 0; j < (KB + 3) / 4; ++j)
+  for (int j = 0; j < KB / 4; ++j)
+  {
+    uint32_t ones = 0, zeros = 0;
+    for (uint32_t o = tid & 31; o < G; o += 32)
     {
-      const uint32_t o = __reduce_or_sync(0xffffffffu, uint32_t((unsigned long long) ones >> (32 * j)));
-      const uint32_t z = __reduce_or_sync(0xffffffffu, uint32_t((unsigned long long) zeros >> (32 * j)));
-      __syncthreads();
-      if (tid < 2)
-      {
-        dscratch[tid] = 0u;
-      }
-      __syncthreads();
-      if ((tid & 31) == 0)
-      {
-        atomicOr(&dscratch[0], o);
-        atomicOr(&dscratch[1], z);
-      }
-      __syncthreads();
-      if (tid == 0)
-      {
-        p.table[b * 4 + j * 2]     = dscratch[0];
-        p.table[b * 4 + j * 2 + 1] = dscratch[1];
-      }
+      ones |= __ldcg(bits + o * (KB / 2) + 2 * j);
+      zeros |= __ldcg(bits + o * (KB / 2) + 2 * j + 1);
     }
-    if (!finish_grid_sync(&p.ctrl->barrier, G, target, p.status))
-    {
-      return;
-    }
+    const uint32_t both = __reduce_or_sync(0xffffffffu, ones) & __reduce_or_sync(0xffffffffu, zeros);
 #pragma unroll
-    for (int j = 0; j < (KB + 3) / 4; ++j)
+    for (int q = 0; q < 4; ++q)
     {
-      digits1 = digits0 = 0u;
-      for (uint32_t o = tid & 31; o < G; o += 32)
-      {
-        digits1 |= __ldcg(p.table + o * 4 + j * 2);
-        digits0 |= __ldcg(p.table + o * 4 + j * 2 + 1);
-      }
-      const uint32_t both = __reduce_or_sync(0xffffffffu, digits1) & __reduce_or_sync(0xffffffffu, digits0);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-      {
-        vary |= ((both >> (8 * q)) & 255u) != 0u ? 1u << (4 * j + q) : 0u;
-      }
-    }
-    // every CTA has read the table before any writes its counts
-    if (!finish_grid_sync(&p.ctrl->barrier, G, target, p.status))
-    {
-      return;
+      vary |= ((both >> (8 * q)) & 255u) != 0u ? 1u << (4 * j + q) : 0u;
     }
   }
   if (vary == 0u)
@@ -1407,92 +1438,99 @@ __device__ __forceinline__ void finish_rest_body(const FinishParams& p)
     V* vdst                   = vbuf[cur ^ 1];
     const int bit             = q * RADIX_BITS;
     cur ^= 1;
-    for (int i = tid; i < NW * R; i += TPB)
-    {
-      whist[i] = 0u;
-    }
-    __syncthreads();
-    for (uint32_t v = v0 + tid; v < v1; v += TPB)
-    {
-      atomicAdd(&whist[extract_digit<U, FP>(encode_key<U>(__ldcg(src + v), p.codec), bit, R - 1u)], 1u);
-    }
-    __syncthreads();
-    if (tid < R)
-    {
-      p.table[b * R + tid] = whist[tid];
-      whist[tid]           = 0u;
-    }
-    if (!finish_grid_sync(&p.ctrl->barrier, G, target, p.status))
-    {
-      return;
-    }
-    if (tid < R)
-    {
-      uint32_t total = 0, below = 0;
-#pragma unroll 8
-      for (uint32_t o = 0; o < G; ++o)
+    const bool ok = phase([&](uint32_t b) {
+      for (int i = tid; i < R; i += TPB)
       {
-        const uint32_t c = __ldcg(p.table + o * R + tid);
-        total += c;
-        below += o < b ? c : 0u;
+        place[i] = 0u;
       }
-      place[tid] = digit_exclusive_scan<R>(total, dscratch, tid) + below;
-    }
-    __syncthreads();
-    for (uint32_t t = v0; t < v1; t += TILE)
-    {
-      const uint32_t valid = min(uint32_t(TILE), v1 - t);
-      const int wofs       = (tid >> 5) * ITEMS * 32 + (tid & 31);
-      U raw[ITEMS], keys[ITEMS];
-#pragma unroll
-      for (int i = 0; i < ITEMS; ++i)
+      __syncthreads();
+      const uint32_t v1 = share_begin(b + 1u);
+      for (uint32_t v = share_begin(b) + tid; v < v1; v += TPB)
       {
-        const uint32_t s = uint32_t(wofs + i * 32);
-        raw[i]           = s < valid ? __ldcg(src + t + s) : U(0);
-        keys[i]          = s < valid ? encode_key<U>(raw[i], p.codec) : U(~U(0)); // padding ranks last
+        atomicAdd(&place[extract_digit<U, FP>(encode_key<U>(__ldcg(src + v), p.codec), bit, R - 1u)], 1u);
       }
-      uint32_t* counts = whist + (tid >> 5) * R;
-      warp_histogram<U, FP, ITEMS>(keys, counts, bit, R - 1u);
       __syncthreads();
       if (tid < R)
       {
-        uint32_t start;
-        const uint32_t total = block_digit_offsets<NW>(whist, dscratch, &start, tid);
-        delta[tid]           = place[tid] - start;
-        place[tid] += total - (tid == R - 1 ? uint32_t(TILE) - valid : 0u);
+        p.table[b * R + tid] = place[tid];
       }
-      __syncthreads();
-      uint32_t pos[ITEMS];
-      warp_rank_stable<U, FP, ITEMS>(keys, pos, counts, bit, R - 1u);
-#pragma unroll
-      for (int i = 0; i < ITEMS; ++i)
-      {
-        const uint32_t s = uint32_t(wofs + i * 32);
-        const uint32_t g = delta[extract_digit<U, FP>(keys[i], bit, R - 1u)] + pos[i];
-        if (s < valid && g < m)
-        {
-          dst[g] = raw[i];
-          if constexpr (VB > 0)
-          {
-            vdst[g] = __ldcg(vsrc + t + s);
-          }
-        }
-      }
-      __syncthreads();
+    })
+    && phase([&](uint32_t b) {
+      const uint32_t v1 = share_begin(b + 1u);
       for (int i = tid; i < NW * R; i += TPB)
       {
         whist[i] = 0u;
       }
+      if (tid < R)
+      {
+        uint32_t total = 0, below = 0;
+#pragma unroll 8
+        for (uint32_t o = 0; o < G; ++o)
+        {
+          const uint32_t c = __ldcg(p.table + o * R + tid);
+          total += c;
+          below += o < b ? c : 0u;
+        }
+        place[tid] = digit_exclusive_scan<R>(total, dscratch, tid) + below;
+      }
       __syncthreads();
-    }
-    if (!finish_grid_sync(&p.ctrl->barrier, G, target, p.status))
+      for (uint32_t t = share_begin(b); t < v1; t += TILE)
+      {
+        const uint32_t valid = min(uint32_t(TILE), v1 - t);
+        const int wofs       = (tid >> 5) * ITEMS * 32 + (tid & 31);
+        U raw[ITEMS], coded[ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+        {
+          const uint32_t s = uint32_t(wofs + i * 32);
+          raw[i]           = s < valid ? __ldcg(src + t + s) : U(0);
+          coded[i]         = s < valid ? encode_key<U>(raw[i], p.codec) : U(~U(0)); // padding ranks last
+        }
+        uint32_t* counts = whist + (tid >> 5) * R;
+        warp_histogram<U, FP, ITEMS>(coded, counts, bit, R - 1u);
+        __syncthreads();
+        if (tid < R)
+        {
+          uint32_t start;
+          const uint32_t total = block_digit_offsets<NW>(whist, dscratch, &start, tid);
+          delta[tid]           = place[tid] - start;
+          place[tid] += total - (tid == R - 1 ? uint32_t(TILE) - valid : 0u);
+        }
+        __syncthreads();
+        uint32_t pos[ITEMS];
+        warp_rank_stable<U, FP, ITEMS>(coded, pos, counts, bit, R - 1u);
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+        {
+          const uint32_t s = uint32_t(wofs + i * 32);
+          const uint32_t g = delta[extract_digit<U, FP>(coded[i], bit, R - 1u)] + pos[i];
+          if (s < valid && g < m)
+          {
+            dst[g] = raw[i];
+            if constexpr (VB > 0)
+            {
+              vdst[g] = __ldcg(vsrc + t + s);
+            }
+          }
+        }
+        __syncthreads();
+        for (int i = tid; i < NW * R; i += TPB)
+        {
+          whist[i] = 0u;
+        }
+        __syncthreads();
+      }
+    });
+    if (!ok)
     {
       return;
     }
   }
   if (!whole)
   {
-    transfer(false, cur);
+    phase([&](uint32_t b) {
+      transfer(b, false, cur);
+    });
   }
 }
 

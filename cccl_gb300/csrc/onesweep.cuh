@@ -15,8 +15,9 @@
 //      values follow the same permutation.
 //
 // Two kernels run these steps:
-//   * onesweep_persistent_body: the main path. One CTA per SM, launched cooperatively, walks
-//     tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the next tile's keys and values are
+//   * onesweep_persistent_body: the main path. One CTA per SM, launched cooperatively where
+//     there are more tiles than CTAs, walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... (one
+//     tile per CTA: the next one by ticket); the next tile's keys and values are
 //     fetched into shared memory by a bulk async copy (cp.async.bulk + mbarrier) while the
 //     current tile is ranked, so HBM latency is off the critical path. Its threads are
 //     split: 256 look-back threads run step 2 while the others rank, and a tile is written
@@ -626,7 +627,7 @@ struct PersistentSmem
   static_assert(MT >= 32 && MT % 32 == 0, "whole main warps");
 };
 // misc words: [2] sticky failure of the CTA (its stores are disabled), [3] single-digit
-// flag and digit of the tile being ranked, [4] digit of the tile's first key, [8..15] scan
+// flag and digit of the tile being ranked, [4] digit of the tile's first key, [5] first tile, [8..15] scan
 // scratch, [16..21] three mbarriers, [22..31] the pass's buffers and flags (PassIO).
 
 // Pass hook of the persistent kernel: the plain radix pass has none. A hook may fill its
@@ -731,9 +732,15 @@ __device__ __forceinline__ void onesweep_persistent_impl(const OnesweepParams& p
     mbar_init(&mbar[2], 1);
     mbar_init_fence();
     misc[2] = 0u;
-    if (blockIdx.x < nfull)
+    // With one tile per CTA the tile is taken by ticket, and the launch need not be cooperative: the
+    // look-back waits only for tiles that a running CTA took. More tiles than CTAs stay in fixed
+    // turns: with tickets for all of them passes took 2 to 5 % longer (GB300; 2^21 to 2^26 items,
+    // u64+u32 and f64+i64 pairs).
+    const uint32_t first = ntiles <= gridDim.x ? atomicAdd(p.tile_counter, 1u) : blockIdx.x;
+    misc[5]              = first;
+    if (first < nfull)
     {
-      issue(blockIdx.x, 0);
+      issue(first, 0);
     }
   }
   for (int i = tid; i < NW * R; i += TPB)
@@ -890,7 +897,7 @@ __device__ __forceinline__ void onesweep_persistent_impl(const OnesweepParams& p
     int prev_buf        = 0;
     uint32_t prev_valid = 0;
     bool have_prev      = false;
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x)
+    for (uint32_t t = misc[5]; t < ntiles; t += gridDim.x)
     {
       const uint32_t tn = t + gridDim.x;
       const int nbuf    = buf == 2 ? 0 : buf + 1;
@@ -1082,7 +1089,7 @@ __device__ __forceinline__ void onesweep_persistent_impl(const OnesweepParams& p
     const int d                = tid - MT; // this thread's digit
     const uint32_t skip_tile   = gb300_fault_skip_tile; // no tile, unless a test withholds one
     const unsigned long long bin_base = p.bins[d]; // the digit's global offset, the same for every tile
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x)
+    for (uint32_t t = misc[5]; t < ntiles; t += gridDim.x)
     {
       const uint32_t valid = min(uint32_t(TILE), p.portion_items - t * TILE);
       asm volatile("bar.sync 3, %0;" ::"n"(TPB) : "memory"); // BH

@@ -21,6 +21,7 @@
   extern "C" __global__ void __launch_bounds__(gb300::ONESWEEP_TPB)                                             \
     gb300_onesweep_dyn_k##KB##_v##VB##_##SUF(const gb300::OnesweepParams p)                                     \
   {                                                                                                             \
+    gb300::wait_for_previous_grid();                                                                            \
     gb300::OnesweepParams q = p;                                                                                \
     if (gb300::apply_pass_plan<KB, VB>(q))                                                                      \
     {                                                                                                           \
@@ -30,6 +31,7 @@
   extern "C" __global__ void __launch_bounds__(gb300::persistent_tpb(KB, VB), gb300::PERSISTENT_MINB)                                        \
     gb300_onesweep_k##KB##_v##VB##_##SUF(const gb300::OnesweepParams p)                                         \
   {                                                                                                             \
+    gb300::wait_for_previous_grid();                                                                            \
     gb300::onesweep_persistent_body<KB, VB, FP, gb300::persistent_tpb(KB, VB), gb300::persistent_items(KB, VB), true>(p); \
   }
 
@@ -40,6 +42,7 @@
   extern "C" __global__ void __launch_bounds__(gb300::persistent_tpb(KB, 0), gb300::PERSISTENT_MINB)                                   \
     gb300_onesweep_first_k##KB##_v0_i(const gb300::OnesweepParams p)                                            \
   {                                                                                                             \
+    gb300::wait_for_previous_grid();                                                                            \
     gb300::onesweep_persistent_body<KB, 0, false, gb300::persistent_tpb(KB, 0), gb300::persistent_items(KB, 0), false>(p); \
   }
 
@@ -47,6 +50,7 @@
   extern "C" __global__ void __launch_bounds__(gb300::SINGLE_TILE_TPB)                                          \
     gb300_single_tile_k##KB##_v##VB##_##SUF(const gb300::SingleTileParams p)                                    \
   {                                                                                                             \
+    gb300::wait_for_previous_grid();                                                                            \
     gb300::single_tile_body<KB, VB, FP, gb300::SINGLE_TILE_TPB, gb300::SINGLE_TILE_ITEMS>(p);                   \
   }
 
@@ -54,6 +58,7 @@
   extern "C" __global__ void __launch_bounds__(gb300::HISTOGRAM_LANES_TPB, 1)                                   \
     gb300_histogram_k##KB##_##SUF(const gb300::HistogramParams p)                                               \
   {                                                                                                             \
+    gb300::wait_for_previous_grid();                                                                            \
     gb300::histogram_lanes_body<KB, FP, gb300::HISTOGRAM_LANES_TPB>(p);                                         \
   }
 
@@ -88,11 +93,13 @@
   extern "C" __global__ void __launch_bounds__(gb300::finish_tpb(KB, VB, false) + 32, gb300::finish_minb(false))  \
     gb300_finish_k##KB##_v##VB##_##SUF(const gb300::FinishParams p)                                               \
   {                                                                                                               \
+    gb300::wait_for_previous_grid();                                                                              \
     gb300::finish_body<KB, VB, FP, false>(p);                                                                     \
   }                                                                                                               \
   extern "C" __global__ void __launch_bounds__(gb300::finish_tpb(KB, VB, true) + 32, gb300::finish_minb(true))    \
     gb300_finish_tail_k##KB##_v##VB##_##SUF(const gb300::FinishParams p)                                          \
   {                                                                                                               \
+    gb300::wait_for_previous_grid();                                                                              \
     if (gb300::gate_open(p.gate) && __ldcg(&p.ctrl->route) != 0u)                                                 \
     {                                                                                                             \
       gb300::finish_body<KB, VB, FP, true>(p);                                                                    \
@@ -107,5 +114,6 @@
 
 extern "C" __global__ void __launch_bounds__(256) gb300_init(const gb300::InitParams p)
 {
+  gb300::wait_for_previous_grid();
   gb300::init_body(p);
 }

@@ -30,7 +30,8 @@ struct RadixPolicy
   int32_t persistent_items;
   int32_t gather_value_bytes; // > 0: the caller's values have this width, sorted as 32-bit indices
   int32_t finish; // 1: the image holds the partition-and-finish kernels (blobs of older builds: 0)
-  int32_t reserved[3];
+  int32_t chained; // 1: the image's kernels wait for the grid before them and take their tiles by ticket
+  int32_t reserved[2];
   uint64_t onesweep_smem;
   uint64_t single_tile_smem;
   uint64_t persistent_smem;

@@ -93,6 +93,15 @@ __device__ __forceinline__ U decode_key(U t, const KeyCodec& c)
   return U(t ^ U((t & high_bit<U>()) ? c.inv_set : c.inv_clr));
 }
 
+// First statement of a kernel that may be launched while the grid before it still runs (chained
+// launches, abi_common.h): waits until that grid has ended and its writes are visible, then
+// lets the next launch of the chain begin its own start. In any other launch it does nothing.
+__device__ __forceinline__ void wait_for_previous_grid()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // False when the kernel is gated off (see KernelGate).
 __device__ __forceinline__ bool gate_open(const KernelGate& g)
 {

@@ -104,6 +104,8 @@ struct InitParams
   KernelGate gate;
 };
 
+constexpr int FINISH_MAX_PHASES = 24; // offsets 2, gather, varying digits, 2 per pass, back
+
 // Partition-and-finish route of a plain sort (finish_kernels.cuh), in the control block;
 // zeroed with it, written by the histogram kernel.
 struct FinishControl
@@ -113,7 +115,7 @@ struct FinishControl
   uint32_t num_pieces;
   uint32_t prefix_shift; // low key bits the partition did not sort by
   uint32_t ticket;       // next piece
-  uint32_t barrier;      // grid-wide barrier of the rest kernel
+  uint32_t large_done;   // large pieces written
   uint32_t large_pieces; // pieces listed in FinishParams::large
   uint32_t large_ticket;
   uint32_t search_step;    // a power of 8
@@ -122,6 +124,9 @@ struct FinishControl
   // sample of the keys' top 1, 2, .. digits (finish_sample)
   unsigned long long light[MAX_PASSES];
   uint32_t heavy[MAX_PASSES];
+  // work of the phases of finish_tail (finish_phase)
+  uint32_t claimed[FINISH_MAX_PHASES];
+  uint32_t done[FINISH_MAX_PHASES];
 };
 
 struct HistogramParams
@@ -169,7 +174,7 @@ struct FinishParams
   FinishRange* rest;  // [num_pieces]: what finish_tail sorts as one sequence (items 0: nothing)
   FinishRange* large; // [num_pieces]: pieces for the general form
   uint32_t* offsets;  // [num_pieces]
-  uint32_t* table;    // [FINISH_MAX_CTAS][256]
+  uint32_t* table;    // [FINISH_MAX_CTAS][256], then [FINISH_MAX_CTAS][4]
   uint32_t* status;
   KeyCodec codec;
   KernelGate gate;
