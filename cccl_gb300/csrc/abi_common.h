@@ -84,6 +84,20 @@ image_ref radix_image(int key_bytes); // one cubin per key width
 image_ref segmented_image(int key_bytes); // one cubin per key width
 image_ref learned_image(int key_bytes);   // 4- and 8-byte keys
 
+// Payload of a build result: the library's own image, which it only points to (copying its 15 MB
+// took 1 ms of a 5 ms build), or a deserialised copy, which it owns.
+inline void free_payload(void* payload)
+{
+  for (int kb : {1, 2, 4, 8})
+  {
+    if (payload == radix_image(kb).data || payload == segmented_image(kb).data)
+    {
+      return;
+    }
+  }
+  delete[] static_cast<char*>(payload);
+}
+
 // ---- key kinds ----
 enum key_kind : int
 {

@@ -132,8 +132,6 @@ try
   const size_t value_size = gathered ? 4 : user_value;
 
   const image_ref img = radix_image(key_bytes);
-  std::unique_ptr<char[]> payload(new char[img.size]);
-  std::memcpy(payload.get(), img.data, img.size);
 
   auto* pol        = static_cast<RadixPolicy*>(std::malloc(sizeof(RadixPolicy)));
   if (pol == nullptr)
@@ -154,7 +152,7 @@ try
 
   cccl_device_radix_sort_build_result_t r{};
   r.cc                   = cc_major * 10 + cc_minor;
-  r.payload              = payload.release();
+  r.payload              = const_cast<void*>(static_cast<const void*>(img.data)); // the library's own (free_payload)
   r.payload_size         = img.size;
   r.payload_kind         = CCCL_PAYLOAD_CUBIN;
   r.key_type             = input_keys_it.value_type;
@@ -526,7 +524,7 @@ try
   {
     return CUDA_ERROR_INVALID_VALUE;
   }
-  delete[] static_cast<char*>(b->payload);
+  free_payload(b->payload);
   b->payload = nullptr;
   std::free(b->runtime_policy);
   b->runtime_policy = nullptr;

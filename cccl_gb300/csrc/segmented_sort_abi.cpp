@@ -55,7 +55,7 @@ bool keys_only(const cccl_iterator_t& values)
 
 void free_result(cccl_device_segmented_sort_build_result_t* b)
 {
-  delete[] static_cast<char*>(b->payload);
+  free_payload(b->payload);
   b->payload = nullptr;
   std::free(b->runtime_policy);
   b->runtime_policy = nullptr;
@@ -275,8 +275,6 @@ try
   const bool gathered = !(user_value == 0 || user_value == 4 || user_value == 8);
   const size_t vb     = gathered ? 4 : user_value;
   const image_ref img = segmented_image(kb);
-  std::unique_ptr<char[]> payload(new char[img.size]);
-  std::memcpy(payload.get(), img.data, img.size);
 
   auto* pol = static_cast<SegmentedPolicy*>(std::malloc(sizeof(SegmentedPolicy)));
   auto* tab = static_cast<SegKernelTable*>(std::calloc(1, sizeof(SegKernelTable)));
@@ -316,7 +314,7 @@ try
 
   cccl_device_segmented_sort_build_result_t r{};
   r.cc                            = cc_major * 10 + cc_minor;
-  r.payload                       = payload.release();
+  r.payload                       = const_cast<void*>(static_cast<const void*>(img.data)); // the library's own (free_payload)
   r.payload_size                  = img.size;
   r.payload_kind                  = CCCL_PAYLOAD_CUBIN;
   r.key_type                      = d_keys_in.value_type;
