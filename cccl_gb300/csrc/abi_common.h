@@ -228,7 +228,15 @@ inline void launch(
 // stream's time. A chain of short kernels takes 1.6 us a launch instead of 4.2 (GB300).
 template <class Params>
 inline void launch_after(
-  const char* role, CUkernel kernel, unsigned grid, unsigned block, size_t smem, CUstream stream, const Params& p, bool chained)
+  const char* role,
+  CUkernel kernel,
+  unsigned grid,
+  unsigned block,
+  size_t smem,
+  CUstream stream,
+  const Params& p,
+  bool chained,
+  unsigned cluster = 1)
 {
   if (!chained)
   {
@@ -241,9 +249,13 @@ inline void launch_after(
     check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
           "cuFuncSetAttribute(max dynamic shared memory)");
   }
-  CUlaunchAttribute attr{};
-  attr.id                                         = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
-  attr.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchAttribute attr[2]{};
+  attr[0].id                                           = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  attr[0].value.programmaticStreamSerializationAllowed = 1;
+  attr[1].id                                           = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+  attr[1].value.clusterDim.x                           = cluster;
+  attr[1].value.clusterDim.y                           = 1;
+  attr[1].value.clusterDim.z                           = 1;
   CUlaunchConfig config{};
   config.gridDimX       = grid;
   config.gridDimY       = 1;
@@ -253,8 +265,8 @@ inline void launch_after(
   config.blockDimZ      = 1;
   config.sharedMemBytes = unsigned(smem);
   config.hStream        = stream;
-  config.attrs          = &attr;
-  config.numAttrs       = 1;
+  config.attrs          = attr;
+  config.numAttrs       = cluster > 1 ? 2 : 1;
   void* args[]          = {const_cast<Params*>(&p)};
   notify_launch(role, 0, stream);
   check(cuLaunchKernelEx(&config, f, args, nullptr), "cuLaunchKernelEx");
@@ -296,6 +308,33 @@ inline int occupancy(CUkernel kernel, int block, size_t smem)
     throw cuda_error(CUDA_ERROR_INVALID_VALUE, "kernel cannot be resident on an SM");
   }
   return n;
+}
+
+// Whether the device can run one cluster of `cluster` CTAs of the kernel (sets the kernel's limits).
+inline bool cluster_fits(CUkernel kernel, unsigned cluster, unsigned block, size_t smem)
+{
+  CUfunction f = function_of(kernel);
+  check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
+        "cuFuncSetAttribute(max dynamic shared memory)");
+  check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_NON_PORTABLE_CLUSTER_SIZE_ALLOWED, 1),
+        "cuFuncSetAttribute(non-portable cluster size)");
+  CUlaunchAttribute attr{};
+  attr.id                 = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+  attr.value.clusterDim.x = cluster;
+  attr.value.clusterDim.y = 1;
+  attr.value.clusterDim.z = 1;
+  CUlaunchConfig config{};
+  config.gridDimX       = cluster;
+  config.gridDimY       = 1;
+  config.gridDimZ       = 1;
+  config.blockDimX      = block;
+  config.blockDimY      = 1;
+  config.blockDimZ      = 1;
+  config.sharedMemBytes = unsigned(smem);
+  config.attrs          = &attr;
+  config.numAttrs       = 1;
+  int n                 = 0;
+  return cuOccupancyMaxActiveClusters(&n, f, &config) == CUDA_SUCCESS && n >= 1;
 }
 
 inline int sm_count()

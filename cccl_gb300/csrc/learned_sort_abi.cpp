@@ -170,6 +170,10 @@ CCCL_GB300_API CUresult cccl_gb300_learned_sort_build(
       ks.onesweep_first         = get_kernel(r.radix_library, nm.onesweep_first);
       ks.onesweep_dyn           = get_kernel(r.radix_library, nm.onesweep_dyn);
       ks.single_tile            = get_kernel(r.radix_library, nm.single_tile);
+      if (pol.cluster == 1)
+      {
+        ks.cluster = get_kernel(r.radix_library, nm.cluster);
+      }
       if (pol.finish == 1)
       {
         ks.finish      = get_kernel(r.radix_library, nm.finish);

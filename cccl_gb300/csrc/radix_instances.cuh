@@ -3,6 +3,7 @@
 // resolves with cuLibraryGetKernel; see kernel_names.h for the naming scheme.
 #pragma once
 
+#include "cluster_kernels.cuh"
 #include "radix_kernels.cuh"
 #include "gather_kernels.cuh"
 #include "merge_kernels.cuh"
@@ -72,7 +73,18 @@
   GB300_SINGLE_TILE(KB, 8, gb300::FP_BLOCK_DESC, fd)    \
   GB300_SINGLE_TILE(KB, 16, gb300::FP_BLOCK_DESC, fd)
 
+#define GB300_CLUSTER_SORT(KB, VB, FP, SUF)                                                                       \
+  extern "C" __global__ void __launch_bounds__(gb300::CLUSTER_TPB, 1)                                             \
+    gb300_cluster_sort_k##KB##_v##VB##_##SUF(const gb300::ClusterSortParams p)                                    \
+  {                                                                                                               \
+    gb300::wait_for_previous_grid();                                                                              \
+    gb300::cluster_sort_body<KB, VB, FP>(p);                                                                      \
+  }
+
 #define GB300_ALL_VALUES(KB, FP, SUF)  \
+  GB300_CLUSTER_SORT(KB, 0, FP, SUF)   \
+  GB300_CLUSTER_SORT(KB, 4, FP, SUF)   \
+  GB300_CLUSTER_SORT(KB, 8, FP, SUF)   \
   GB300_ONESWEEP(KB, 0, FP, SUF)       \
   GB300_ONESWEEP(KB, 1, FP, SUF)       \
   GB300_ONESWEEP(KB, 2, FP, SUF)       \

@@ -35,6 +35,7 @@ RadixPolicy make_radix_policy(int key_bytes, int value_bytes, int key_kind)
   p.persistent_smem   = persistent_smem_bytes(key_bytes, value_bytes);
   p.single_tile_smem  = single_tile_smem_bytes(key_bytes);
   p.chained           = 1;
+  p.cluster           = cluster_supported(key_bytes, value_bytes) ? 1 : 0;
   p.finish            = finish_supported(key_bytes, value_bytes) ? 1 : 0;
   return p;
 }
@@ -51,6 +52,10 @@ RadixKernelNames radix_kernel_names(int kb, int vb, int kind, bool descending)
   n.onesweep_first = (vb == 0 && kind != KIND_FLOAT) ? "gb300_onesweep_first_" + kv : n.onesweep;
   // descending float sorts: CUB's single tile folds -0.0 into +0.0 before ordering (FP_BLOCK_DESC)
   n.single_tile = "gb300_single_tile_" + (kind == KIND_FLOAT && descending ? kv + "d" : kv);
+  if (cluster_supported(kb, vb))
+  {
+    n.cluster = "gb300_cluster_sort_" + kv;
+  }
   if (finish_supported(kb, vb))
   {
     n.finish      = "gb300_finish_" + kv;
@@ -272,6 +277,33 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
   // buffers that are not 16-byte aligned take every pass (the finish bulk-copies its pieces)
   const bool finish = t.finish && persistent && ks.finish != nullptr;
   auto* fctrl       = reinterpret_cast<FinishControl*>(base + t.finish_ctrl_off);
+
+  // Short sorts: one cluster, one launch. The temporary storage is only used for the status word.
+  if (pol.cluster == 1 && ks.cluster != nullptr && n <= cluster_max_items(kb, vb))
+  {
+    const int ipt     = int(ceil_div(n, uint64_t(CLUSTER_CTAS) * CLUSTER_TPB));
+    const size_t smem = cluster_smem_bytes(kb, vb, ipt);
+    if (cluster_fits(ks.cluster, CLUSTER_CTAS, CLUSTER_TPB, smem))
+    {
+      const int result = c.overwrite ? passes & 1 : 1; // the buffer that the passes would end in
+      ClusterSortParams p{};
+      p.keys_in          = c.keys[0];
+      p.keys_out         = c.keys[result];
+      p.values_in        = has_vals ? c.values[0] : nullptr;
+      p.values_out       = has_vals ? c.values[result] : nullptr;
+      p.status           = &ctrl->status;
+      p.num_items        = uint32_t(n);
+      p.items_per_thread = uint32_t(ipt);
+      p.tile_magic       = uint32_t(ceil_div(uint64_t(1) << 32, uint64_t(CLUSTER_TPB) * ipt));
+      p.begin_bit        = c.begin_bit;
+      p.end_bit          = c.end_bit;
+      p.codec            = codec;
+      p.gate             = c.gate;
+      launch_after("cluster_sort", ks.cluster, CLUSTER_CTAS, CLUSTER_TPB, smem, c.stream, p, true, CLUSTER_CTAS);
+      *selector = passes & 1;
+      return;
+    }
+  }
 
   // 1. zero the control block (histogram counters, tile counters, status)
   {

@@ -31,7 +31,8 @@ struct RadixPolicy
   int32_t gather_value_bytes; // > 0: the caller's values have this width, sorted as 32-bit indices
   int32_t finish; // 1: the image holds the partition-and-finish kernels (blobs of older builds: 0)
   int32_t chained; // 1: the image's kernels wait for the grid before them and take their tiles by ticket
-  int32_t reserved[2];
+  int32_t cluster; // 1: the image has the cluster sort's kernels
+  int32_t reserved[1];
   uint64_t onesweep_smem;
   uint64_t single_tile_smem;
   uint64_t persistent_smem;
@@ -49,6 +50,7 @@ struct RadixKernels
   CUkernel single_tile;
   CUkernel finish; // partition and finish (finish_kernels.cuh); unused unless RadixPolicy::finish
   CUkernel finish_tail;
+  CUkernel cluster; // short sorts (cluster_kernels.cuh); unused unless RadixPolicy::cluster
 };
 
 // Kernel names of one (key width, value width, key kind) in the radix image.
@@ -56,6 +58,7 @@ struct RadixKernelNames
 {
   std::string init, histogram, onesweep, onesweep_first, onesweep_dyn, single_tile;
   std::string finish, finish_tail; // empty where the finish does not carry the types
+  std::string cluster;             // likewise
 };
 RadixKernelNames radix_kernel_names(int key_bytes, int value_bytes, int key_kind, bool descending);
 

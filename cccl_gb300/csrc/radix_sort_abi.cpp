@@ -164,7 +164,7 @@ try
   const bool fin = pol->finish == 1;
   r.upsweep_kernel_lowered_name                = dup_cstr(fin ? names.finish : his);
   r.alt_upsweep_kernel_lowered_name            = dup_cstr(fin ? names.finish_tail : his);
-  r.scan_bins_kernel_lowered_name              = dup_cstr(his);
+  r.scan_bins_kernel_lowered_name              = dup_cstr(pol->cluster == 1 ? names.cluster : his);
   r.downsweep_kernel_lowered_name              = dup_cstr(dyn);
   r.alt_downsweep_kernel_lowered_name          = dup_cstr(first);
   r.histogram_kernel_lowered_name              = dup_cstr(his);
@@ -350,7 +350,8 @@ CCCL_C_API CUresult cccl_device_radix_sort(
                     build.downsweep_kernel,
                     build.single_tile_kernel,
                     build.upsweep_kernel,
-                    build.alt_upsweep_kernel};
+                    build.alt_upsweep_kernel,
+                    build.scan_bins_kernel};
     RadixCall call{};
     call.keys[0]          = d_keys_in.state;
     call.keys[1]          = d_keys_out.state;

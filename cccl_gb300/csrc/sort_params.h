@@ -215,6 +215,22 @@ struct OnesweepParams
   const uint32_t* plan_prev;
 };
 
+struct ClusterSortParams
+{
+  const void* keys_in;
+  void* keys_out; // may be keys_in
+  const void* values_in;
+  void* values_out;
+  uint32_t* status;
+  uint32_t num_items;
+  uint32_t items_per_thread;
+  uint32_t tile_magic; // ceil(2^32 / (CLUSTER_TPB * items_per_thread))
+  int begin_bit;
+  int end_bit;
+  KeyCodec codec;
+  KernelGate gate;
+};
+
 struct SingleTileParams
 {
   const void* keys_in;

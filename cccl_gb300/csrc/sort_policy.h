@@ -155,6 +155,40 @@ GB300_HD constexpr unsigned long long persistent_tile_items(int tpb, int items)
   return (unsigned long long) (tpb - LOOKBACK_THREADS) * items;
 }
 
+// Short sorts by one cluster (cluster_kernels.cuh): sixteen CTAs, the largest cluster, keep the
+// items in their registers and, twice, in shared memory.
+constexpr int CLUSTER_CTAS = 16;
+constexpr int CLUSTER_TPB  = 1024;
+
+GB300_HD constexpr bool cluster_supported(int kb, int vb)
+{
+  return (void) kb, vb == 0 || vb == 4 || vb == 8;
+}
+
+GB300_HD constexpr size_t cluster_smem_bytes(int kb, int vb, int items_per_thread)
+{
+  return size_t(4) * (256 * (CLUSTER_TPB / 32 + 2 * CLUSTER_CTAS + CLUSTER_TPB / 256 + 2) + 16)
+       + size_t(2) * (kb + vb) * CLUSTER_TPB * items_per_thread;
+}
+
+// Items per thread, at most: 48 bytes of keys and values. The cluster's time grows with the bytes
+// that cross it, that of the launches it replaces hardly does up to one tile per SM. A sort on
+// GB300 by the cluster and by the launches: 98304 f32+u32 44.8 and 46.5 us (131072: 51.4), 65536
+// u64+u32 71.6 and 78 (98304: 78.9), 49152 f64+i64 71.6 and 73, 131072 u32 36.8 and 43.
+GB300_HD constexpr int cluster_items(int kb, int vb)
+{
+  return 48 / (kb + vb) < 8 ? 48 / (kb + vb) : 8;
+}
+static_assert(cluster_smem_bytes(4, 4, cluster_items(4, 4)) <= 227 * 1024
+                && cluster_smem_bytes(8, 4, cluster_items(8, 4)) <= 227 * 1024
+                && cluster_smem_bytes(8, 8, cluster_items(8, 8)) <= 227 * 1024,
+              "a cluster CTA's items fit its shared memory");
+
+GB300_HD constexpr unsigned long long cluster_max_items(int kb, int vb)
+{
+  return (unsigned long long) CLUSTER_CTAS * CLUSTER_TPB * cluster_items(kb, vb);
+}
+
 // PLAN_* words of a plain sort's digit passes (see sort_params.h) from the passes whose
 // digit is the same for every key (bit q of trivial_mask). Runs on the device (one thread
 // of the histogram's last CTA) and on the host (the CPU test of every mask).
