@@ -11,7 +11,8 @@
 //     cub/cub/block/block_merge_sort.cuh:39-160,425-520, cub/cub/thread/thread_sort.cuh:27-50)
 //     with the key type's own operator<; this is what decides where NaN keys land, so it
 //     is reproduced step for step;
-//   * block class: one CTA sorts the segment in shared memory with stable 8-bit passes;
+//   * block class: one CTA sorts the segment in shared memory with stable 8-bit passes, or, up to 512
+//     keys of up to 4 bytes, one warp in its registers (warp_sort.cuh);
 //   * device class: all large segments together run the onesweep machinery, one launch per
 //     digit pass over every large segment's tiles, each segment with its own look-back
 //     chain and digit bases (CUB sorts each large segment with a single CTA,
@@ -25,14 +26,10 @@
 #include "block_merge.cuh"
 #include "onesweep.cuh"
 #include "radix_kernels.cuh"
+#include "warp_sort.cuh"
 
 namespace gb300
 {
-
-__device__ __forceinline__ long long load_offset(const void* p, unsigned long long i, int wide)
-{
-  return wide ? static_cast<const long long*>(p)[i] : (long long) static_cast<const int*>(p)[i];
-}
 
 // Appends `item` to list[counter] with one atomic per warp and list.
 __device__ __forceinline__ void warp_append(bool take, uint32_t* counter, uint32_t* list, uint32_t item)
@@ -612,6 +609,22 @@ __device__ __forceinline__ void seg_block_body(const SegSortParams& p, const uin
                                               p.end_bit,
                                               p.codec);
     }
+  }
+}
+
+// The shortest block class: one warp per segment for keys of up to 4 bytes (warp_sort.cuh), one CTA
+// for wider ones.
+template <int KB, int VB, int FP, int TPB, int ITEMS, int BITS>
+__device__ __forceinline__ void seg_block_xs_body(const SegSortParams& p)
+{
+  if constexpr (KB <= 4)
+  {
+    static_assert(TPB * ITEMS <= WARP_SORT_MAX, "the class's longest segment fits a warp");
+    seg_warp_body<KB, VB, FP, TPB>(p, p.block_xs_list, SEG_CTR_BLOCK_XS);
+  }
+  else
+  {
+    seg_block_body<KB, VB, FP, TPB, ITEMS, BITS>(p, p.block_xs_list, SEG_CTR_BLOCK_XS, SEG_CTR_TICKET_BLOCK_XS);
   }
 }
 

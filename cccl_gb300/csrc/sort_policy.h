@@ -546,10 +546,10 @@ GB300_HD constexpr int seg_block_l_tpb(int kb)
 {
   return SEG_BLOCK_L_CAP / seg_block_l_items(kb);
 }
-// block_xs: segments longer than the medium network's tile and up to 512 keys, one CTA of
-// 256 threads x 2 keys each (one thread per digit, as every block pass needs). Small
-// registers and shared memory keep eight CTAs resident per SM (four-byte keys), against four
-// or five of block_s, whose 2048-key tile would be mostly padding for these segments.
+// block_xs: segments longer than the medium network's tile and up to 512 keys. Keys of up to 4 bytes:
+// one warp per segment (warp_sort.cuh), four CTAs of eight warps per SM. 8-byte keys: one CTA of
+// 256 threads x 2 keys each (one thread per digit, as every block pass needs), six per SM; block_s's
+// 2048-key tile would be mostly padding for these segments.
 constexpr int SEG_BLOCK_XS_CAP = 512;
 GB300_HD constexpr int seg_block_xs_items(int kb)
 {
@@ -564,7 +564,7 @@ GB300_HD constexpr int seg_block_xs_minb(int kb)
 #ifdef GB300_SEG_BLOCK_XS_MINB
   return (void) kb, GB300_SEG_BLOCK_XS_MINB;
 #else
-  return kb == 8 ? 6 : 8;
+  return kb == 8 ? 6 : 4; // up to 4 bytes: 16 elements of 8 bytes a lane, 64 registers
 #endif
 }
 constexpr int SEG_NETWORK_TPB   = 256;

@@ -1,0 +1,275 @@
+// Sort of a short segment by one warp, in registers: the shortest block class of the segmented sort
+// for keys of up to 4 bytes.
+//
+// Lane l holds elements l * E to l * E + E - 1 of a bitonic network of 32 * E elements, E = 4, 8 or 16
+// by the segment's length. Every merge starts with the mirrored comparison (element i of a block of k
+// with element k - 1 - i), so all comparisons point the same way; comparisons inside a lane are a
+// minimum and a maximum, those across lanes a shuffle, a comparison and a select.
+//   * integer keys alone, ordered by all their bits: the keys themselves are sorted. Equal keys are
+//     the same bytes, so no stability is needed.
+//   * else the elements are the digit window above the source index: distinct, and in the order that
+//     stable digit passes give. The raw keys wait in shared memory, the values in the input.
+//
+// What bounds it: instruction issue, 2 to 3 instructions a slot and lane for the keys themselves, no
+// barrier of the CTA and no pass over shared memory but the transposition in front of the
+// coalesced stores. Sixteen million i32 keys in rows of about 200: 106 us, 442 with one CTA and four
+// digit passes a segment; the class's share of 2^27 f32+i32 in uneven segments: 86 us, was 116.
+#pragma once
+
+#include "radix_kernels.cuh"
+
+namespace gb300
+{
+
+__device__ __forceinline__ long long load_offset(const void* p, unsigned long long i, int wide)
+{
+  return wide ? static_cast<const long long*>(p)[i] : (long long) static_cast<const int*>(p)[i];
+}
+
+// Sorts the 32 * E elements of the warp.
+template <class T, int E>
+__device__ __forceinline__ void warp_bitonic_sort(T (&x)[E])
+{
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 2; k <= 32 * E; k *= 2)
+  {
+    // element i with element k - 1 - i of its block of k
+    if (k <= E)
+    {
+#pragma unroll
+      for (int r = 0; r < E; ++r)
+      {
+        const int o = (r & ~(k - 1)) | (k - 1 - (r & (k - 1)));
+        if (r < o)
+        {
+          const T a = x[r], b = x[o];
+          const bool less = a < b;
+          x[r]            = less ? a : b;
+          x[o]            = less ? b : a;
+        }
+      }
+    }
+    else
+    {
+      const bool upper = (lane & (k / E / 2)) != 0; // keeps the larger one
+#pragma unroll
+      for (int r = 0; r < E / 2; ++r)
+      {
+        const T a  = __shfl_xor_sync(0xffffffffu, x[E - 1 - r], k / E - 1);
+        const T b  = __shfl_xor_sync(0xffffffffu, x[r], k / E - 1);
+        x[r]         = (x[r] < a) != upper ? x[r] : a;
+        x[E - 1 - r] = (x[E - 1 - r] < b) != upper ? x[E - 1 - r] : b;
+      }
+    }
+    // then with the element j behind it, j = k / 4, k / 8, ...
+#pragma unroll
+    for (int j = k / 4; j >= 1; j /= 2)
+    {
+      if (j < E)
+      {
+#pragma unroll
+        for (int r = 0; r < E; ++r)
+        {
+          if ((r & j) == 0)
+          {
+            const T a = x[r], b = x[r | j];
+            const bool less = a < b;
+            x[r]            = less ? a : b;
+            x[r | j]        = less ? b : a;
+          }
+        }
+      }
+      else
+      {
+        const bool upper = (lane & (j / E)) != 0;
+#pragma unroll
+        for (int r = 0; r < E; ++r)
+        {
+          const T a = __shfl_xor_sync(0xffffffffu, x[r], j / E);
+          x[r]      = (x[r] < a) != upper ? x[r] : a;
+        }
+      }
+    }
+  }
+}
+
+// Place of element i in the warp's transposition buffer: one word of padding per 32, so lanes E
+// elements apart (a power of two) and lanes one element apart both reach 32 banks.
+__device__ __forceinline__ int warp_sort_slot(int i)
+{
+  return i + (i >> 5);
+}
+
+constexpr int WARP_SORT_MAX   = 512;                            // elements
+constexpr int WARP_SORT_SLOTS = WARP_SORT_MAX + WARP_SORT_MAX / 32;
+
+template <int KB>
+struct WarpSortSmem
+{
+  union
+  {
+    uint32_t keys[WARP_SORT_SLOTS]; // sorted keys on their way out
+    struct
+    {
+      uint16_t order[WARP_SORT_SLOTS]; // sorted source indices
+      typename uint_of<KB>::type raw[WARP_SORT_MAX];
+    } pairs;
+  };
+};
+
+template <int KB, int VB, int FP, int E>
+__device__ __forceinline__ void warp_sort_segment(
+  const typename uint_of<KB>::type* kin,
+  typename uint_of<KB>::type* kout,
+  const typename value_word<VB>::type* vin,
+  typename value_word<VB>::type* vout,
+  int n,
+  int begin_bit,
+  int end_bit,
+  const KeyCodec& codec,
+  WarpSortSmem<KB>& sh)
+{
+  using U        = typename uint_of<KB>::type;
+  using V        = typename value_word<VB>::type;
+  const int lane = threadIdx.x & 31;
+  __syncwarp(); // the previous segment's reads of sh are done
+  if (VB == 0 && FP == FP_NONE && begin_bit == 0 && end_bit == 8 * KB)
+  {
+    uint32_t x[E];
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      const int i = r * 32 + lane;
+      x[r]        = i < n ? uint32_t(encode_key<U>(kin[i], codec)) : ~0u;
+    }
+    warp_bitonic_sort<uint32_t, E>(x);
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      sh.keys[warp_sort_slot(lane * E + r)] = x[r];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      const int i = r * 32 + lane;
+      if (i < n)
+      {
+        kout[i] = decode_key<U>(U(sh.keys[warp_sort_slot(i)]), codec);
+      }
+    }
+  }
+  else
+  {
+    using T = typename uint_of<(KB <= 2 ? 4 : 8)>::type; // window and index
+    constexpr int SHIFT  = KB <= 2 ? 16 : 32;
+    const uint32_t dmask = end_bit - begin_bit >= 32 ? ~0u : (1u << (end_bit - begin_bit)) - 1u;
+    T x[E];
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      const int i = r * 32 + lane;
+      if (i < n)
+      {
+        const U k          = kin[i];
+        sh.pairs.raw[i]    = k;
+        const uint32_t key = (uint32_t(digit_source<U, FP>(encode_key<U>(k, codec))) >> begin_bit) & dmask;
+        x[r]               = T(T(key) << SHIFT) | T(i);
+      }
+      else
+      {
+        x[r] = T(~T(0)); // above every element: an index has fewer bits than the space below the key
+      }
+    }
+    warp_bitonic_sort<T, E>(x);
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      sh.pairs.order[warp_sort_slot(lane * E + r)] = uint16_t(x[r]);
+    }
+    __syncwarp();
+    uint32_t from[E];
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      const int i = r * 32 + lane;
+      from[r]     = i < n ? min(uint32_t(sh.pairs.order[warp_sort_slot(i)]), uint32_t(n - 1)) : 0u;
+    }
+    if constexpr (VB > 0)
+    {
+      // all of them before the first store: input and output may be one buffer
+      V v[E];
+#pragma unroll
+      for (int r = 0; r < E; ++r)
+      {
+        v[r] = vin[from[r]];
+      }
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < E; ++r)
+      {
+        if (r * 32 + lane < n)
+        {
+          vout[r * 32 + lane] = v[r];
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      if (r * 32 + lane < n)
+      {
+        kout[r * 32 + lane] = sh.pairs.raw[from[r]];
+      }
+    }
+  }
+}
+
+// Every warp takes the list's segments in fixed turns: their lengths differ by a factor of four at
+// most, and a ticket per segment would be one atomic on one address for 500 bytes of keys.
+template <int KB, int VB, int FP, int TPB>
+__device__ __forceinline__ void seg_warp_body(const SegSortParams& p, const uint32_t* list, uint32_t count_index)
+{
+  using U = typename uint_of<KB>::type;
+  using V = typename value_word<VB>::type;
+  __shared__ WarpSortSmem<KB> smem[TPB / 32];
+  WarpSortSmem<KB>& sh = smem[threadIdx.x / 32];
+  const uint32_t count = p.counters[count_index];
+  const uint32_t step  = gridDim.x * (TPB / 32);
+  uint32_t item        = blockIdx.x * (TPB / 32) + threadIdx.x / 32;
+  long long b = 0, e = 0;
+  auto segment = [&](uint32_t i) {
+    if (i < count)
+    {
+      const uint32_t s = list[i];
+      b                = load_offset(p.begin_offsets, s, p.offsets_64);
+      e                = load_offset(p.end_offsets, s, p.offsets_64);
+    }
+  };
+  segment(item);
+  for (; item < count; item += step)
+  {
+    const long long first = b;
+    const int n           = int(min(e - b, (long long) WARP_SORT_MAX));
+    segment(item + step); // its offsets arrive while this one is sorted
+    const U* kin = static_cast<const U*>(p.keys_in) + first;
+    U* kout      = static_cast<U*>(p.keys_out) + first;
+    const V* vin = VB > 0 ? static_cast<const V*>(p.values_in) + first : nullptr;
+    V* vout      = VB > 0 ? static_cast<V*>(p.values_out) + first : nullptr;
+    if (n <= 128)
+    {
+      warp_sort_segment<KB, VB, FP, 4>(kin, kout, vin, vout, n, p.begin_bit, p.end_bit, p.codec, sh);
+    }
+    else if (n <= 256)
+    {
+      warp_sort_segment<KB, VB, FP, 8>(kin, kout, vin, vout, n, p.begin_bit, p.end_bit, p.codec, sh);
+    }
+    else
+    {
+      warp_sort_segment<KB, VB, FP, 16>(kin, kout, vin, vout, n, p.begin_bit, p.end_bit, p.codec, sh);
+    }
+  }
+}
+
+} // namespace gb300
