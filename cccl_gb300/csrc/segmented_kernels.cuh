@@ -628,6 +628,25 @@ __device__ __forceinline__ void seg_block_xs_body(const SegSortParams& p)
   }
 }
 
+// Segments of up to 2048 keys. 4-byte integer keys alone, ordered by all their bits, by a group of
+// warps (warp_sort.cuh), the others by one CTA and digit passes (narrower keys take only one or two).
+template <int KB, int VB, int FP, int TPB, int ITEMS, int BITS>
+__device__ __forceinline__ void seg_block_s_body(const SegSortParams& p)
+{
+  if constexpr (KB == 4 && VB == 0 && FP == FP_NONE)
+  {
+    static_assert(TPB * ITEMS <= GROUP_SORT_MAX, "the class's longest segment fits a group");
+    static_assert(sizeof(uint32_t) * WARP_SORT_SLOTS * (TPB / 32) <= block_sort_smem(KB, TPB, ITEMS),
+                  "the groups' exchange fits the class's shared memory");
+    if (p.begin_bit == 0 && p.end_bit == 8 * KB)
+    {
+      seg_group_body<KB, TPB>(p, p.block_s_list, SEG_CTR_BLOCK_S);
+      return;
+    }
+  }
+  seg_block_body<KB, VB, FP, TPB, ITEMS, BITS>(p, p.block_s_list, SEG_CTR_BLOCK_S, SEG_CTR_TICKET_BLOCK_S);
+}
+
 // ---------------------------------------------------------------------------------------
 // device class: all large segments together
 // ---------------------------------------------------------------------------------------

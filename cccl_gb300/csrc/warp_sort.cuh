@@ -26,71 +26,81 @@ __device__ __forceinline__ long long load_offset(const void* p, unsigned long lo
   return wide ? static_cast<const long long*>(p)[i] : (long long) static_cast<const int*>(p)[i];
 }
 
-// Sorts the 32 * E elements of the warp.
-template <class T, int E>
-__device__ __forceinline__ void warp_bitonic_sort(T (&x)[E])
+// Compares every element with the one J behind it, then J / 2, ... 1.
+template <class T, int E, int J>
+__device__ __forceinline__ void warp_bitonic_merge(T (&x)[E])
 {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int k = 2; k <= 32 * E; k *= 2)
+  for (int j = J; j >= 1; j /= 2)
   {
-    // element i with element k - 1 - i of its block of k
-    if (k <= E)
+    if (j < E)
     {
 #pragma unroll
       for (int r = 0; r < E; ++r)
       {
-        const int o = (r & ~(k - 1)) | (k - 1 - (r & (k - 1)));
-        if (r < o)
+        if ((r & j) == 0)
         {
-          const T a = x[r], b = x[o];
+          const T a = x[r], b = x[r | j];
           const bool less = a < b;
           x[r]            = less ? a : b;
-          x[o]            = less ? b : a;
+          x[r | j]        = less ? b : a;
         }
       }
     }
     else
     {
-      const bool upper = (lane & (k / E / 2)) != 0; // keeps the larger one
+      const bool upper = (lane & (j / E)) != 0; // keeps the larger one
 #pragma unroll
-      for (int r = 0; r < E / 2; ++r)
+      for (int r = 0; r < E; ++r)
       {
-        const T a  = __shfl_xor_sync(0xffffffffu, x[E - 1 - r], k / E - 1);
-        const T b  = __shfl_xor_sync(0xffffffffu, x[r], k / E - 1);
-        x[r]         = (x[r] < a) != upper ? x[r] : a;
-        x[E - 1 - r] = (x[E - 1 - r] < b) != upper ? x[E - 1 - r] : b;
+        const T a = __shfl_xor_sync(0xffffffffu, x[r], j / E);
+        x[r]      = (x[r] < a) != upper ? x[r] : a;
       }
     }
-    // then with the element j behind it, j = k / 4, k / 8, ...
+  }
+}
+
+// Sorts blocks of K elements of the warp whose halves are sorted, then of 2 K, ... 32 * E.
+template <class T, int E, int K = 2>
+__device__ __forceinline__ void warp_bitonic_sort(T (&x)[E])
+{
+  const int lane = threadIdx.x & 31;
+  // element i with element K - 1 - i of its block
+  if constexpr (K <= E)
+  {
 #pragma unroll
-    for (int j = k / 4; j >= 1; j /= 2)
+    for (int r = 0; r < E; ++r)
     {
-      if (j < E)
+      const int o = (r & ~(K - 1)) | (K - 1 - (r & (K - 1)));
+      if (r < o)
       {
-#pragma unroll
-        for (int r = 0; r < E; ++r)
-        {
-          if ((r & j) == 0)
-          {
-            const T a = x[r], b = x[r | j];
-            const bool less = a < b;
-            x[r]            = less ? a : b;
-            x[r | j]        = less ? b : a;
-          }
-        }
-      }
-      else
-      {
-        const bool upper = (lane & (j / E)) != 0;
-#pragma unroll
-        for (int r = 0; r < E; ++r)
-        {
-          const T a = __shfl_xor_sync(0xffffffffu, x[r], j / E);
-          x[r]      = (x[r] < a) != upper ? x[r] : a;
-        }
+        const T a = x[r], b = x[o];
+        const bool less = a < b;
+        x[r]            = less ? a : b;
+        x[o]            = less ? b : a;
       }
     }
+  }
+  else
+  {
+    const bool upper = (lane & (K / E / 2)) != 0;
+#pragma unroll
+    for (int r = 0; r < E / 2; ++r)
+    {
+      const T a    = __shfl_xor_sync(0xffffffffu, x[E - 1 - r], K / E - 1);
+      const T b    = __shfl_xor_sync(0xffffffffu, x[r], K / E - 1);
+      x[r]         = (x[r] < a) != upper ? x[r] : a;
+      x[E - 1 - r] = (x[E - 1 - r] < b) != upper ? x[E - 1 - r] : b;
+    }
+  }
+  if constexpr (K >= 4)
+  {
+    warp_bitonic_merge<T, E, K / 4>(x);
+  }
+  if constexpr (K < 32 * E)
+  {
+    warp_bitonic_sort<T, E, 2 * K>(x);
   }
 }
 
@@ -101,7 +111,8 @@ __device__ __forceinline__ int warp_sort_slot(int i)
   return i + (i >> 5);
 }
 
-constexpr int WARP_SORT_MAX   = 512;                            // elements
+constexpr int WARP_SORT_MAX   = 512; // elements
+constexpr int GROUP_SORT_MAX  = 4 * WARP_SORT_MAX;
 constexpr int WARP_SORT_SLOTS = WARP_SORT_MAX + WARP_SORT_MAX / 32;
 
 template <int KB>
@@ -222,6 +233,113 @@ __device__ __forceinline__ void warp_sort_segment(
       {
         kout[r * 32 + lane] = sh.pairs.raw[from[r]];
       }
+    }
+  }
+}
+
+// Integer keys alone, ordered by all their bits: a segment by a group of four warps, 32 * E elements a
+// warp, warp by warp. Each warp sorts its own, then the warps merge two by two: the steps across
+// warps through shared memory (each warp's part of `sh`), the rest within them. `bar` (1 or 2) is the
+// group's named barrier.
+template <int KB, int E>
+__device__ __forceinline__ void group_sort_segment(
+  const typename uint_of<KB>::type* kin,
+  typename uint_of<KB>::type* kout,
+  int n,
+  const KeyCodec& codec,
+  uint32_t (*sh)[WARP_SORT_SLOTS],
+  int bar)
+{
+  using U          = typename uint_of<KB>::type;
+  constexpr int W  = 4;
+  constexpr int WE = 32 * E; // elements of a warp
+  const int lane   = threadIdx.x & 31;
+  const int warp   = (threadIdx.x >> 5) % W;
+  auto sync        = [&]() {
+    // constant barrier numbers: a number in a register claims all of the CTA's barriers
+    if (bar == 1)
+    {
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory");
+    }
+    else
+    {
+      asm volatile("bar.sync 2, %0;" ::"n"(32 * W) : "memory");
+    }
+  };
+  uint32_t x[E];
+#pragma unroll
+  for (int r = 0; r < E; ++r)
+  {
+    const int i = warp * WE + r * 32 + lane;
+    x[r]        = i < n ? uint32_t(encode_key<U>(kin[i], codec)) : ~0u;
+  }
+  warp_bitonic_sort<uint32_t, E>(x);
+  // element i of this warp with element i of warp `other`, or (mirrored) with element WE - 1 - i
+  auto exchange = [&](int other, bool mirrored) {
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      sh[warp][warp_sort_slot(lane * E + r)] = x[r];
+    }
+    sync();
+#pragma unroll
+    for (int r = 0; r < E; ++r)
+    {
+      const int i      = lane * E + r;
+      const uint32_t a = sh[other][warp_sort_slot(mirrored ? WE - 1 - i : i)];
+      x[r]             = warp < other ? min(x[r], a) : max(x[r], a);
+    }
+    sync(); // before the next writes
+  };
+  exchange(warp ^ 1, true);
+  warp_bitonic_merge<uint32_t, E, WE / 2>(x);
+  exchange(warp ^ 3, true);
+  exchange(warp ^ 1, false);
+  warp_bitonic_merge<uint32_t, E, WE / 2>(x);
+#pragma unroll
+  for (int r = 0; r < E; ++r)
+  {
+    sh[warp][warp_sort_slot(lane * E + r)] = x[r];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < E; ++r)
+  {
+    const int i = warp * WE + r * 32 + lane;
+    if (i < n)
+    {
+      kout[i] = decode_key<U>(U(sh[warp][warp_sort_slot(r * 32 + lane)]), codec);
+    }
+  }
+  __syncwarp();
+}
+
+// block_s with keys alone: two groups of four warps a CTA, a segment of up to 2048 keys each. The
+// groups take the list's segments in fixed turns.
+template <int KB, int TPB>
+__device__ __forceinline__ void seg_group_body(const SegSortParams& p, const uint32_t* list, uint32_t count_index)
+{
+  using U              = typename uint_of<KB>::type;
+  constexpr int GROUPS = TPB / 128;
+  static_assert(GROUPS == 2, "named barriers 1 and 2");
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int group      = threadIdx.x / 128;
+  auto* sh             = reinterpret_cast<uint32_t(*)[WARP_SORT_SLOTS]>(smem) + 4 * group;
+  const uint32_t count = p.counters[count_index];
+  for (uint32_t item = blockIdx.x * GROUPS + group; item < count; item += gridDim.x * GROUPS)
+  {
+    const uint32_t s  = list[item];
+    const long long b = load_offset(p.begin_offsets, s, p.offsets_64);
+    const int n       = int(min(load_offset(p.end_offsets, s, p.offsets_64) - b, (long long) GROUP_SORT_MAX));
+    const U* kin      = static_cast<const U*>(p.keys_in) + b;
+    U* kout           = static_cast<U*>(p.keys_out) + b;
+    if (n <= GROUP_SORT_MAX / 2)
+    {
+      group_sort_segment<KB, 8>(kin, kout, n, p.codec, sh, 1 + group);
+    }
+    else
+    {
+      group_sort_segment<KB, 16>(kin, kout, n, p.codec, sh, 1 + group);
     }
   }
 }
