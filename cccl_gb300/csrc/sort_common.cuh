@@ -102,6 +102,26 @@ __device__ __forceinline__ void wait_for_previous_grid()
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The same for a kernel that may run beside the launches before it, up to the last one with
+// how == CHAIN_WAIT (that one has started, so what it waited for is over): it does its work at once
+// and waits before it ends, so that whoever waits for it has waited for those too.
+__device__ __forceinline__ void chain_begin(int how)
+{
+  if (how != CHAIN_BESIDE)
+  {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ void chain_end(int how)
+{
+  if (how == CHAIN_BESIDE)
+  {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+}
+
 // False when the kernel is gated off (see KernelGate).
 __device__ __forceinline__ bool gate_open(const KernelGate& g)
 {

@@ -309,6 +309,10 @@ struct SegClassifyParams
   int pad1;
 };
 
+// How a kernel of a chained launch starts (chain_begin in sort_common.cuh)
+constexpr int CHAIN_WAIT   = 0; // when the launch before it has ended
+constexpr int CHAIN_BESIDE = 1; // at once
+
 struct SegSortParams
 {
   const void* keys_in;
@@ -328,6 +332,7 @@ struct SegSortParams
   KeyCodec codec;
   int begin_bit; // key bits the block classes sort by
   int end_bit;
+  int chain; // CHAIN_*
 };
 
 struct SegDeviceParams
@@ -352,6 +357,7 @@ struct SegDeviceParams
   uint32_t* lookback[2];
   uint32_t* status;
   KeyCodec codec;
+  int chain; // CHAIN_*, of the histogram
 };
 
 // ---- stable merge of two sorted runs (merge_kernels.cuh) ----
