@@ -82,6 +82,20 @@ struct PassIO
   int decode_out;
 };
 
+// Whether this kernel runs the pass, of two launched for it (OnesweepParams::turn): the order-free
+// one if the plan makes it the first that runs, else the stable one, which also does what a
+// skipped pass has to.
+__device__ __forceinline__ bool pass_turn(const OnesweepParams& p)
+{
+  if (p.turn == PASS_ALONE)
+  {
+    return true;
+  }
+  const uint32_t w = __ldcg(p.plan);
+  const bool first = (w & PLAN_SKIP) == 0u && (w & PLAN_ENCODE) != 0u;
+  return first == (p.turn == PASS_IF_FIRST);
+}
+
 // Resolves the pass's buffers. Returns false when the pass does nothing: gated off, or
 // skipped by its plan (its digit is the same for every key), in which case the grid first
 // clears this portion's rows of the next pass's look-back buffer, as the pass would have,

@@ -33,7 +33,10 @@
     gb300_onesweep_k##KB##_v##VB##_##SUF(const gb300::OnesweepParams p)                                         \
   {                                                                                                             \
     gb300::wait_for_previous_grid();                                                                            \
-    gb300::onesweep_persistent_body<KB, VB, FP, gb300::persistent_tpb(KB, VB), gb300::persistent_items(KB, VB), true>(p); \
+    if (gb300::pass_turn(p))                                                                                    \
+    {                                                                                                           \
+      gb300::onesweep_persistent_body<KB, VB, FP, gb300::persistent_tpb(KB, VB), gb300::persistent_items(KB, VB), true>(p); \
+    }                                                                                                           \
   }
 
 // First pass of a full-width integer keys-only sort: equal digits may land in any order
@@ -44,7 +47,10 @@
     gb300_onesweep_first_k##KB##_v0_i(const gb300::OnesweepParams p)                                            \
   {                                                                                                             \
     gb300::wait_for_previous_grid();                                                                            \
-    gb300::onesweep_persistent_body<KB, 0, false, gb300::persistent_tpb(KB, 0), gb300::persistent_items(KB, 0), false>(p); \
+    if (gb300::pass_turn(p))                                                                                    \
+    {                                                                                                           \
+      gb300::onesweep_persistent_body<KB, 0, false, gb300::persistent_tpb(KB, 0), gb300::persistent_items(KB, 0), false>(p); \
+    }                                                                                                           \
   }
 
 #define GB300_SINGLE_TILE(KB, VB, FP, SUF)                                                                        \

@@ -180,6 +180,11 @@ struct FinishParams
   KernelGate gate;
 };
 
+// A digit pass may be launched twice, once for each form (pass_turn in onesweep.cuh)
+constexpr uint32_t PASS_ALONE        = 0;
+constexpr uint32_t PASS_IF_FIRST     = 1; // the order-free form
+constexpr uint32_t PASS_IF_NOT_FIRST = 2; // the stable form
+
 struct OnesweepParams
 {
   const void* keys_in;        // portion-relative
@@ -191,7 +196,7 @@ struct OnesweepParams
   uint32_t portion_items;
   uint32_t portion_tiles;
   uint32_t tile_row_base;     // first look-back row of this portion
-  uint32_t pad0;
+  uint32_t turn;              // PASS_*
   uint32_t* lookback;         // [row][digit] for this pass
   uint32_t* lookback_next;    // buffer of the next pass; this pass zeroes its rows
   uint32_t* tile_counter;
