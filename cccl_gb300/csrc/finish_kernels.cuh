@@ -36,17 +36,6 @@ __device__ __forceinline__ U finish_prefix(U raw, const KeyCodec& c, int shift)
   return U(digit_source<U, FP>(encode_key<U>(raw, c)) >> shift);
 }
 
-__device__ __forceinline__ unsigned long long finish_mix(unsigned long long x)
-{
-  // 64-bit finaliser of MurmurHash3 (Austin Appleby, public domain)
-  x ^= x >> 33;
-  x *= 0xff51afd7ed558ccdull;
-  x ^= x >> 33;
-  x *= 0xc4ceb9fe1a85ec53ull;
-  x ^= x >> 33;
-  return x;
-}
-
 // ---------------------------------------------------------------------------------------
 // Sample: how large the buckets of the top `level` digits are. One CTA of the histogram
 // kernel per level counts the groups of equal prefixes among p.sample_items keys, taken one
@@ -60,6 +49,36 @@ __device__ __forceinline__ unsigned long long finish_mix(unsigned long long x)
 // compare-and-swap it took 26 us with the keys' state in registers, 23 us with it in shared memory.
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t FINISH_NO_SLOT = 0xffffffffu;
+
+// The choice for one set of trivial digits, by one thread.
+template <int KB>
+__device__ __noinline__ uint32_t finish_digits(const HistogramParams& p, uint32_t trivial_mask, uint32_t* piece)
+{
+  const FinishControl* f = p.finish;
+  unsigned long long light[8];
+  uint32_t heavy[8];
+  for (int l = 0; l < KB; ++l)
+  {
+    light[l] = __ldcg(&f->light[l]);
+    heavy[l] = __ldcg(&f->heavy[l]);
+  }
+  return uint32_t(finish_choose(KB, trivial_mask, light, heavy, p.num_items, p.sample_items, p.finish_cap, p.finish_cost,
+                                p.plan_mode, piece));
+}
+
+// A level is sampled: the thread that counts the last one makes the choice for no trivial digit.
+template <int KB>
+__device__ __forceinline__ void finish_sampled(const HistogramParams& p)
+{
+  __threadfence();
+  if (atomicAdd(&p.finish->levels_done, 1u) + 1u == uint32_t(p.sample_levels))
+  {
+    __threadfence();
+    uint32_t piece           = 0;
+    p.finish->sampled_digits = finish_digits<KB>(p, 0u, &piece);
+    p.finish->sampled_piece  = piece;
+  }
+}
 
 template <int KB, int FP, int TPB>
 __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned char* smem, int level)
@@ -145,6 +164,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
         if (tid == 0)
         {
           p.finish->heavy[level - 1] = uint32_t((unsigned long long) heavy * samples / TPB);
+          finish_sampled<KB>(p);
         }
         __syncthreads(); // the shared memory is the histogram's again
         return;          // uniform
@@ -184,26 +204,21 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   {
     p.finish->light[level - 1] = light_sum;
     p.finish->heavy[level - 1] = heavy_sum;
+    finish_sampled<KB>(p);
   }
   __syncthreads(); // the shared memory is the histogram's again
 }
 
 // Route of the sort, by one thread of the histogram's last CTA. Returns the digits below
-// the partition as extra skippable passes (0: the LSD route).
+// the partition as extra skippable passes (0: the LSD route). With no trivial digit the choice is
+// the one that the last sampling CTA made while the others counted (finish_sampled): it takes
+// 3 us, and every other CTA would wait for it here.
 template <int KB>
 __device__ __noinline__ uint32_t finish_route(const HistogramParams& p, uint32_t trivial_mask)
 {
-  FinishControl* f = p.finish;
-  unsigned long long light[8];
-  uint32_t heavy[8];
-  for (int l = 0; l < KB; ++l)
-  {
-    light[l] = __ldcg(&f->light[l]);
-    heavy[l] = __ldcg(&f->heavy[l]);
-  }
-  uint32_t piece   = 0;
-  const int digits = finish_choose(KB, trivial_mask, light, heavy, p.num_items, p.sample_items, p.finish_cap,
-                                   p.finish_cost, p.plan_mode, &piece);
+  FinishControl* f      = p.finish;
+  uint32_t piece        = __ldcg(&f->sampled_piece);
+  const uint32_t digits = trivial_mask == 0u ? __ldcg(&f->sampled_digits) : finish_digits<KB>(p, trivial_mask, &piece);
   if (digits == 0)
   {
     return 0u;

@@ -351,13 +351,22 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
       };
       p.sample_heavy       = heavy(mean);
       p.sample_heavy_first = heavy(mean * HISTOGRAM_LANES_TPB / p.sample_items);
-      // The sampling CTAs count keys too only where that takes longer than the sample (keys of
-      // more than 2^30 bytes); below, the other CTAs are done before they would be.
+      // The sampling CTAs count keys too where that takes longer than the sample, from the trip on at
+      // which the others get there; below, the others are done before they would be.
       const unsigned sms    = unsigned(sm_count());
       const unsigned levels = unsigned(kb);
-      if (n * uint64_t(kb) <= (1ull << 30) && grid + levels > sms)
+      if (grid + levels > sms)
       {
-        grid = sms - levels;
+        const uint64_t rows = n * kb / (16 * uint64_t(HISTOGRAM_LANES_TPB)); // 16-byte loads of a CTA
+        const uint64_t lead = HISTOGRAM_LEAD_TRIPS;
+        if (rows >= 4 * lead * (sms - levels) + 4 * sms)
+        {
+          p.lead_trips = uint32_t(lead);
+        }
+        else
+        {
+          grid = std::min(grid, sms - levels);
+        }
       }
       p.hist_ctas = int(grid);
       grid        = std::min(grid + levels, sms);

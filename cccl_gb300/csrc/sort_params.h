@@ -119,7 +119,7 @@ struct FinishControl
   uint32_t large_pieces; // pieces listed in FinishParams::large
   uint32_t large_ticket;
   uint32_t search_step;    // a power of 8
-  uint32_t pad;
+  uint32_t levels_done;    // levels sampled
   unsigned long long rest_items;
   // sample of the keys' top 1, 2, .. digits (finish_sample)
   unsigned long long light[MAX_PASSES];
@@ -127,6 +127,8 @@ struct FinishControl
   // work of the phases of finish_tail (finish_phase)
   uint32_t claimed[FINISH_MAX_PHASES];
   uint32_t done[FINISH_MAX_PHASES];
+  uint32_t sampled_digits; // the choice when no digit is trivial
+  uint32_t sampled_piece;
 };
 
 struct HistogramParams
@@ -153,6 +155,7 @@ struct HistogramParams
   uint32_t sample_heavy_first; // the same for the first 2^10 sampled keys alone
   uint32_t finish_cap;        // largest piece the finish's first launch takes
   float finish_cost;          // time of the finish, in digit passes
+  uint32_t lead_trips; // trips of the counting CTAs before the sampling ones join (histogram_lanes_count)
 };
 
 // Pieces of the partitioned array (finish_kernels.cuh).

@@ -245,6 +245,8 @@ constexpr int FINISH_BIN_MAX        = 64;      // keys of a bin that the common 
 constexpr int FINISH_KNOTS          = 32;      // stretches of a large piece's bins
 constexpr int FINISH_SMALLEST_PIECE = 2;       // piece_items is at least CAP / 2
 constexpr int FINISH_REST_ITEMS     = 4;
+// Trips of the histogram's CTAs before those that sample join: the sample takes about 20 us.
+constexpr int HISTOGRAM_LEAD_TRIPS = 16;
 constexpr unsigned long long FINISH_ORDER_FREE_ITEMS = 1ull << 26; // partition with an order-free first pass
 constexpr int FINISH_MAX_CTAS       = 304;     // shares of the rest
 
