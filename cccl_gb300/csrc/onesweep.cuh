@@ -641,7 +641,7 @@ struct PersistentSmem
   static_assert(MT >= 32 && MT % 32 == 0, "whole main warps");
 };
 // misc words: [2] sticky failure of the CTA (its stores are disabled), [3] single-digit
-// flag and digit of the tile being ranked, [4] digit of the tile's first key, [5] first tile, [8..15] scan
+// flag and digit of the tile being ranked, [4] digit of the tile's first key, [5] first tile less the CTA's number, [8..15] scan
 // scratch, [16..21] three mbarriers, [22..31] the pass's buffers and flags (PassIO).
 
 // Pass hook of the persistent kernel: the plain radix pass has none. A hook may fill its
@@ -751,7 +751,7 @@ __device__ __forceinline__ void onesweep_persistent_impl(const OnesweepParams& p
     // turns: with tickets for all of them passes took 2 to 5 % longer (GB300; 2^21 to 2^26 items,
     // u64+u32 and f64+i64 pairs).
     const uint32_t first = ntiles <= gridDim.x ? atomicAdd(p.tile_counter, 1u) : blockIdx.x;
-    misc[5]              = first;
+    misc[5]              = first - blockIdx.x; // the loops keep their own, uniform, tile number
     if (first < nfull)
     {
       issue(first, 0);
@@ -911,9 +911,10 @@ __device__ __forceinline__ void onesweep_persistent_impl(const OnesweepParams& p
     int prev_buf        = 0;
     uint32_t prev_valid = 0;
     bool have_prev      = false;
-    for (uint32_t t = misc[5]; t < ntiles; t += gridDim.x)
+    for (uint32_t turn = blockIdx.x; turn < ntiles; turn += gridDim.x)
     {
-      const uint32_t tn = t + gridDim.x;
+      const uint32_t t  = turn + misc[5];
+      const uint32_t tn = turn + gridDim.x;
       const int nbuf    = buf == 2 ? 0 : buf + 1;
       if (tid == 0 && tn < nfull)
       {
@@ -1103,8 +1104,10 @@ __device__ __forceinline__ void onesweep_persistent_impl(const OnesweepParams& p
     const int d                = tid - MT; // this thread's digit
     const uint32_t skip_tile   = gb300_fault_skip_tile; // no tile, unless a test withholds one
     const unsigned long long bin_base = p.bins[d]; // the digit's global offset, the same for every tile
-    for (uint32_t t = misc[5]; t < ntiles; t += gridDim.x)
+    const uint32_t shift = misc[5];
+    for (uint32_t turn = blockIdx.x; turn < ntiles; turn += gridDim.x)
     {
+      const uint32_t t     = turn + shift;
       const uint32_t valid = min(uint32_t(TILE), p.portion_items - t * TILE);
       asm volatile("bar.sync 3, %0;" ::"n"(TPB) : "memory"); // BH
       uint32_t start;
