@@ -11,7 +11,8 @@ from segments import edge_segments
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = [57, 112, 113, 127, 128, 129, 255, 256, 257, 300, 511, 512, 513, 700, 1023, 1024, 1025, 1500, 2047, 2048, 2049]
+LENGTHS = [1, 2, 18, 19, 31, 32, 33, 57, 63, 64, 65, 112, 113, 127, 128, 129, 255, 256, 257, 300, 511, 512, 513]
+LENGTHS += [700, 1023, 1024, 1025, 1500, 2047, 2048, 2049]
 TYPES = [
     (np.int32, None),
     (np.uint32, None),
@@ -59,3 +60,13 @@ def test_lengths(oracle, dtype, value, spread, bits):
             ok[lo:hi] = True
         assert ko[ok].tobytes() == rk[ok].tobytes()
         assert v is None or vo[ok].tobytes() == rv[ok].tobytes()
+
+
+def test_few_segments(oracle):
+    """Too few segments to split the short ones into classes."""
+    b, e, n = edge_segments([1, 3, 17, 33, 100, 200, 400, 2000, 3000], gap=3)
+    k = I.uniform_bits(np.uint32, n, np.random.default_rng(22))
+    rk, _ = oracle.segmented_sort(k, None, b, e, descending=False, threads=8)
+    ko, _, _ = gpu_seg_sort(k, None, b, e)
+    for lo, hi in zip(b, e):
+        assert ko[lo:hi].tobytes() == rk[lo:hi].tobytes()
