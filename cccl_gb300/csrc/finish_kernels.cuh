@@ -93,7 +93,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   U* sampled             = reinterpret_cast<U*>(smem + 4 * size_t(slots)); // [samples], later every key's slot
   __shared__ uint32_t light_sum, heavy_sum;
   // one key per stratum of num_items / samples keys, at a hashed place in it
-  const uint32_t width = uint32_t(p.num_items / samples); // >= 1; fewer than 2^30 items
+  const uint32_t width = uint32_t(p.num_items / samples); // >= 1
 #pragma unroll 1
   for (uint32_t i = tid; i < samples; i += TPB)
   {

@@ -86,9 +86,10 @@ plan_radix_temp(const RadixPolicy& pol, uint64_t n, int begin_bit, int end_bit, 
                                                uint64_t(pol.onesweep_tpb) * pol.onesweep_items);
   const uint64_t lookback_rows = ceil_div(n, min_tile) + t.num_portions;
 
-  // Partition and finish: whole keys, one portion (its indices have 32 bits), enough items.
+  // Partition and finish: whole keys, enough items, and few enough for its 32-bit places (with room
+  // for a piece or a search step behind the last).
   t.finish = pol.finish == 1 && begin_bit == 0 && end_bit == 8 * pol.key_bytes && n >= finish_min_items(pol.key_bytes)
-          && t.num_portions == 1;
+          && n < (1ull << 31);
 
   size_t off     = 0;
   t.ctrl_off     = off;

@@ -149,3 +149,30 @@ def test_replayed_from_a_graph(oracle):
         assert _route(temp, 8)[0] == route
         rk, rv = oracle.radix_sort(keys, I.index_values(n), threads=8)
         assert from_dev(ko, np.uint64).tobytes() == rk.tobytes() and from_dev(vo, np.uint32).tobytes() == rv.tobytes()
+
+
+def test_two_portions():
+    """More than 2^30 keys: the partition's passes run as two portions, and places in the pieces go
+    beyond 2^30. A bucket of different keys at the array's end goes to the rest."""
+    import torch
+    from cccl_gb300 import SortOrder, make_radix_sort, sort_status
+    from gpu_util import check_sorted_pairs
+
+    n = (1 << 30) + 12345
+    torch.cuda.empty_cache()
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    k = torch.empty(n, dtype=torch.int64, device="cuda")
+    k.random_(-(1 << 63), (1 << 63) - 1, generator=gen)
+    k[12345 : n : 50] = k[12345 : n : 50] & 0xFFFFFFFFFF | (0x7FFF1234 << 32 & ~0xFFFFFFFFFF)
+    v = torch.arange(n, dtype=torch.int32, device="cuda")
+    ko, vo = torch.empty_like(k), torch.empty_like(v)
+    args = dict(d_in_keys=k, d_out_keys=ko, d_in_values=v, d_out_values=vo)
+    s = make_radix_sort(order=SortOrder.ASCENDING, **args)
+    temp = torch.empty(s(temp_storage=None, num_items=n, **args), dtype=torch.uint8, device="cuda")
+    s(temp_storage=temp, num_items=n, **args)
+    torch.cuda.synchronize()
+    sort_status(temp)
+    route, rest = _route(temp, 8 * 2)
+    assert route == 1 and rest > 0
+    del temp
+    assert check_sorted_pairs(k, ko, vo, "i")
