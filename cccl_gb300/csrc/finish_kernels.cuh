@@ -38,14 +38,15 @@ __device__ __forceinline__ U finish_prefix(U raw, const KeyCodec& c, int shift)
 
 // ---------------------------------------------------------------------------------------
 // Sample: how large the buckets of the top `level` digits are. One CTA of the histogram
-// kernel per level counts the groups of equal prefixes among p.sample_items keys, taken one
-// per stratum, in an open-addressing table in shared memory (word = 17 bits of a 32-bit hash
+// kernel per level counts the groups of equal prefixes among p.sample_items keys
+// (finish_sample_place), in an open-addressing table in shared memory (word = 17 bits of a 32-bit hash
 // of the prefix << 15 | count; 14 other bits choose the slot).
 // Written: the sum of (group size - 1) over the sampled keys of small groups, from which the
 // mean bucket size follows, and the number of sampled keys in groups of at least
 // p.sample_heavy keys, whose buckets the finish cannot take.
-// It delays the histogram by 8 us for 4096 keys: a shared-memory access of all its threads
-// takes 100 clocks (a compare-and-swap 250), so a key costs few of them. In rounds of stores without
+// It takes 8 us for 4096 keys, 20 us for 8192 beside the count (histogram_lanes_count): a
+// shared-memory access of all its threads takes 100 clocks (a compare-and-swap 250), so a key costs
+// few of them. In rounds of stores without
 // compare-and-swap it took 26 us with the keys' state in registers, 23 us with it in shared memory.
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t FINISH_NO_SLOT = 0xffffffffu;
@@ -92,12 +93,12 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   uint32_t* table        = reinterpret_cast<uint32_t*>(smem);          // [slots]
   U* sampled             = reinterpret_cast<U*>(smem + 4 * size_t(slots)); // [samples], later every key's slot
   __shared__ uint32_t light_sum, heavy_sum;
-  // one key per stratum of num_items / samples keys, at a hashed place in it
-  const uint32_t width = uint32_t(p.num_items / samples); // >= 1
+  const uint32_t n = uint32_t(p.num_items); // below 2^31
+  const int half   = finish_sample_half(n);
 #pragma unroll 1
   for (uint32_t i = tid; i < samples; i += TPB)
   {
-    const U* src = keys + ((unsigned long long) width * i + __umulhi((i + 1u) * 0x9e3779b1u, width));
+    const U* src = keys + finish_sample_place(i, n, half);
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(sampled + i)), "l"(src), "n"(KB) : "memory");
   }
 #pragma unroll 1
@@ -117,6 +118,8 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   for (uint32_t i = tid; i < samples; i += TPB)
   {
     const unsigned long long x = finish_prefix<U, FP>(sampled[i], p.codec, shift);
+    // the words mixed by odd multipliers, then a 32-bit finaliser of Chris Wellons' hash-prospector list
+    // (public domain): 15 2c1b3c6d 12 297a2d39 15
     uint32_t h = uint32_t(x) * 0x9e3779b1u + uint32_t(x >> 32) * 0x85ebca77u + 0x27d4eb2fu;
     h          = (h ^ (h >> 15)) * 0x2c1b3c6du;
     h          = (h ^ (h >> 12)) * 0x297a2d39u;

@@ -290,8 +290,7 @@ void segmented_sort_dispatch(const SegmentedPolicy& pol, const SegmentedKernels&
   }
   // 3. warp and block classes: straight from the input into the final buffer. They work on different
   // segments: each starts as soon as the one before has, on the SMs that one leaves free, and so
-  // does the device class's histogram (16.8 M i32 in short rows:
-  // 270 -> 215 us).
+  // does the device class's histogram (16.8 M i32 in short rows: 270 -> 215 us).
   const int beside = chained ? CHAIN_BESIDE : CHAIN_WAIT;
   {
     SegSortParams p{};
@@ -331,9 +330,11 @@ void segmented_sort_dispatch(const SegmentedPolicy& pol, const SegmentedKernels&
     launch_after("seg_block_xs", ks.k[SK_BLOCK_XS], unsigned(sms * occupancy(ks.k[SK_BLOCK_XS], xs_tpb, xs_smem)),
                  unsigned(xs_tpb), xs_smem, c.stream, p, chained);
     launch_after("seg_block_s", ks.k[SK_BLOCK_S],
-                 unsigned(sms * occupancy(ks.k[SK_BLOCK_S], pol.block_s_tpb, pol.block_s_smem)), unsigned(pol.block_s_tpb), pol.block_s_smem, c.stream, p, chained);
+                 unsigned(sms * occupancy(ks.k[SK_BLOCK_S], pol.block_s_tpb, pol.block_s_smem)), unsigned(pol.block_s_tpb),
+                 pol.block_s_smem, c.stream, p, chained);
     launch_after("seg_block_l", ks.k[SK_BLOCK_L],
-                 unsigned(sms * occupancy(ks.k[SK_BLOCK_L], pol.block_l_tpb, pol.block_l_smem)), unsigned(pol.block_l_tpb), pol.block_l_smem, c.stream, p, chained);
+                 unsigned(sms * occupancy(ks.k[SK_BLOCK_L], pol.block_l_tpb, pol.block_l_smem)), unsigned(pol.block_l_tpb),
+                 pol.block_l_smem, c.stream, p, chained);
   }
   // 4. device class: every large segment together, one launch per digit pass
   if (max_dev > 0)

@@ -1,7 +1,7 @@
 // Sort of a short segment by one warp, in registers: the shortest block class of the segmented sort
 // for keys of up to 4 bytes.
 //
-// Lane l holds elements l * E to l * E + E - 1 of a bitonic network of 32 * E elements, E = 4, 8 or 16
+// Lane l holds elements l * E to l * E + E - 1 of a bitonic network (Batcher) of 32 * E elements, E = 4, 8 or 16
 // by the segment's length. Every merge starts with the mirrored comparison (element i of a block of k
 // with element k - 1 - i), so all comparisons point the same way; comparisons inside a lane are a
 // minimum and a maximum, those across lanes a shuffle, a comparison and a select.

@@ -4,6 +4,9 @@
 #include <cstdio>
 #include <initializer_list>
 
+#include <algorithm>
+#include <vector>
+
 #include "sort_policy.h"
 
 using namespace gb300;
@@ -83,6 +86,35 @@ int main()
         std::printf("shape of %d + %d bytes\n", kb, vb);
         ++failures;
       }
+    }
+  }
+  // The places sampled: distinct, inside the array, and spread at random: as many pairs of neighbours
+  // (within a stretch of n / samples places) as independent places have, within five deviations.
+  for (uint32_t n : {(1u << 22), (1u << 22) + 1u, 5000011u, 100000007u, 1u << 28, (1u << 30) + 12345u, (1u << 31) - 1u})
+  {
+    const uint32_t samples = finish_sample_items(n);
+    const int half         = finish_sample_half(n);
+    std::vector<uint32_t> at;
+    for (uint32_t i = 0; i < samples; ++i)
+    {
+      at.push_back(finish_sample_place(i, n, half));
+    }
+    std::sort(at.begin(), at.end());
+    const uint32_t width = n / samples;
+    double pairs         = 0;
+    for (size_t i = 0, j = 0; i < at.size(); i = j)
+    {
+      for (j = i; j < at.size() && at[j] / width == at[i] / width; ++j)
+      {
+      }
+      pairs += 0.5 * double(j - i) * double(j - i - 1);
+    }
+    const double expected = 0.5 * samples;
+    if (at.back() >= n || std::adjacent_find(at.begin(), at.end()) != at.end()
+        || (pairs - expected) * (pairs - expected) > 25 * expected)
+    {
+      std::printf("places of %u: %g pairs, %g expected\n", n, pairs, expected);
+      ++failures;
     }
   }
   std::printf("%d failures\n", failures);

@@ -176,3 +176,32 @@ def test_two_portions():
     assert route == 1 and rest > 0
     del temp
     assert check_sorted_pairs(k, ko, vo, "i")
+
+
+@pytest.mark.parametrize("dist", ["uniform", "normal"])
+def test_sorted_input_is_sampled_fairly(dist):
+    """The sample sees the buckets of keys that are already in order as it does those of the same
+    keys in any order, so the finish is left no large buckets."""
+    import torch
+    from cccl_gb300 import SortOrder, make_radix_sort
+    from gpu_util import check_sorted_pairs
+
+    n = (1 << 26) + 3
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    k = torch.empty(n, dtype=torch.float64, device="cuda")
+    k = k.normal_(generator=gen) if dist == "normal" else k.uniform_(generator=gen)
+    light = []
+    for keys in (k, torch.sort(k)[0]):
+        v = torch.arange(n, dtype=torch.int32, device="cuda")
+        ko, vo = torch.empty_like(keys), torch.empty_like(v)
+        args = dict(d_in_keys=keys, d_out_keys=ko, d_in_values=v, d_out_values=vo)
+        s = make_radix_sort(order=SortOrder.ASCENDING, **args)
+        temp = torch.empty(s(temp_storage=None, num_items=n, **args), dtype=torch.uint8, device="cuda")
+        s(temp_storage=temp, num_items=n, **args)
+        torch.cuda.synchronize()
+        at = (16432 + 4 * 8 + 255) // 256 * 256
+        light.append(temp[at + 48 : at + 48 + 64].cpu().numpy().view(np.uint64).astype(np.int64))
+        assert _route(temp, 8) == (1, 0)
+        assert check_sorted_pairs(keys, ko, vo, "f")
+    # pairs of three digits: some thousand, the same but for their spread
+    assert abs(light[0][2] - light[1][2]) < 12 * np.sqrt(light[0][2]) + 12
