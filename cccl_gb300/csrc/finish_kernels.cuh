@@ -39,8 +39,8 @@ __device__ __forceinline__ U finish_prefix(U raw, const KeyCodec& c, int shift)
 // ---------------------------------------------------------------------------------------
 // Sample: how large the buckets of the top `level` digits are. One CTA of the histogram
 // kernel per level counts the groups of equal prefixes among p.sample_items keys
-// (finish_sample_place), in an open-addressing table in shared memory (word = 17 bits of a 32-bit hash
-// of the prefix << 15 | count; 14 other bits choose the slot).
+// (finish_sample_place), in an open-addressing table in shared memory (word = 18 bits of a 32-bit hash
+// of the prefix << 14 | count; the other 14 choose the slot).
 // Written: the sum of (group size - 1) over the sampled keys of small groups, from which the
 // mean bucket size follows, and the number of sampled keys in groups of at least
 // p.sample_heavy keys, whose buckets the finish cannot take.
@@ -124,7 +124,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
     h          = (h ^ (h >> 15)) * 0x2c1b3c6du;
     h          = (h ^ (h >> 12)) * 0x297a2d39u;
     h ^= h >> 15;
-    const uint32_t print = h & 0xffff8000u;
+    const uint32_t print = h & 0xffffc000u;
     uint32_t s           = (h ^ (h >> 17)) & (slots - 1u);
     // four places, in a table half full at most: the few keys that find none count as single ones
     uint32_t slot = FINISH_NO_SLOT;
@@ -140,7 +140,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
           break;
         }
       }
-      if ((w & 0xffff8000u) == print)
+      if ((w & 0xffffc000u) == print)
       {
         atomicAdd(table + s, 1u); // at most 2^13 keys
         slot = s;
@@ -155,7 +155,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
       // large groups is settled by them, and counting the others would be a long queue at few
       // counters.
       __syncthreads();
-      const uint32_t many = __popc(__ballot_sync(0xffffffffu, slot != FINISH_NO_SLOT && (table[slot] & 0x7fffu) >= limit));
+      const uint32_t many = __popc(__ballot_sync(0xffffffffu, slot != FINISH_NO_SLOT && (table[slot] & 0x3fffu) >= limit));
       if ((tid & 31) == 0)
       {
         atomicAdd(&heavy_sum, many);
@@ -182,7 +182,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   for (uint32_t i = tid; i < samples; i += TPB)
   {
     const uint32_t slot = reinterpret_cast<uint32_t*>(sampled)[i * (KB / 4)];
-    const uint32_t c    = slot != FINISH_NO_SLOT ? table[slot] & 0x7fffu : 1u;
+    const uint32_t c    = slot != FINISH_NO_SLOT ? table[slot] & 0x3fffu : 1u;
     // Whole keys: a few keys that fill large groups of their own (zeros) do not matter, many keys
     // with several copies do. light: groups of 2 and 3, heavy: the other keys of all small groups
     // (what equal keys add to light at the other levels).
