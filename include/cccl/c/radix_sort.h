@@ -23,8 +23,9 @@
  *      upsweep_kernel, alt_upsweep_kernel  whole 4- and 8-byte keys with values of 0, 4 or 8
  *                                    bytes: the two kernels that finish a sort partitioned by its
  *                                    top digits; else the histogram kernel
- *      scan_bins_kernel              the histogram kernel (CUB's multi-pass kernels are never
- *                                    used on sm_90+), so that the member is non-null
+ *      scan_bins_kernel              values of 0, 4 or 8 bytes: the sort of short inputs by one
+ *                                    cluster; else the histogram kernel (CUB's multi-pass kernels
+ *                                    are never used on sm_90+), so that the member is non-null
  *  - runtime_policy: the tile configuration chosen for the key/value types.
  */
 #pragma once
