@@ -205,18 +205,35 @@ inline CUfunction function_of(CUkernel k)
 using launch_observer_fn = void (*)(void*, const char*, int, CUstream);
 void notify_launch(const char* role, int phase, CUstream stream);
 
-template <class Params>
-inline void launch(
-  const char* role, CUkernel kernel, unsigned grid, unsigned block, size_t smem, CUstream stream, const Params& p)
+// Dynamic shared memory that a kernel may be launched with. The limit is the kernel's, and threads
+// that sort with one build share the kernel: every call sets the same value, what the kernel's largest
+// launch takes, since one that set its own size could lower the limit between another's setting and
+// its launch, which would then be refused.
+inline void allow_smem(CUfunction f, size_t most)
 {
-  CUfunction f = function_of(kernel);
-  // dynamic shared memory near the 48 KB default leaves no room for a kernel's static shared
-  // memory: opt in above 47 KB
-  if (smem > 47 * 1024)
+  // near the 48 KB default no room is left for a kernel's static shared memory: opt in above 47 KB
+  if (most > 47 * 1024)
   {
-    check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
+    check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(most)),
           "cuFuncSetAttribute(max dynamic shared memory)");
   }
+}
+
+// most_smem, here and below: of the kernel's largest launch, where launches differ in smem (0: all
+// launches of the kernel take smem).
+template <class Params>
+inline void launch(
+  const char* role,
+  CUkernel kernel,
+  unsigned grid,
+  unsigned block,
+  size_t smem,
+  CUstream stream,
+  const Params& p,
+  size_t most_smem = 0)
+{
+  CUfunction f = function_of(kernel);
+  allow_smem(f, most_smem > smem ? most_smem : smem);
   void* args[] = {const_cast<Params*>(&p)};
   notify_launch(role, 0, stream);
   check(cuLaunchKernel(f, grid, 1, 1, block, 1, 1, unsigned(smem), stream, args, nullptr), "cuLaunchKernel");
@@ -236,19 +253,16 @@ inline void launch_after(
   CUstream stream,
   const Params& p,
   bool chained,
+  size_t most_smem = 0,
   unsigned cluster = 1)
 {
   if (!chained)
   {
-    launch(role, kernel, grid, block, smem, stream, p);
+    launch(role, kernel, grid, block, smem, stream, p, most_smem);
     return;
   }
   CUfunction f = function_of(kernel);
-  if (smem > 47 * 1024)
-  {
-    check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
-          "cuFuncSetAttribute(max dynamic shared memory)");
-  }
+  allow_smem(f, most_smem > smem ? most_smem : smem);
   CUlaunchAttribute attr[2]{};
   attr[0].id                                           = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
   attr[0].value.programmaticStreamSerializationAllowed = 1;
@@ -280,11 +294,7 @@ inline void launch_cooperative(
   const char* role, CUkernel kernel, unsigned grid, unsigned block, size_t smem, CUstream stream, const Params& p)
 {
   CUfunction f = function_of(kernel);
-  if (smem > 48 * 1024)
-  {
-    check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
-          "cuFuncSetAttribute(max dynamic shared memory)");
-  }
+  allow_smem(f, smem);
   void* args[] = {const_cast<Params*>(&p)};
   notify_launch(role, 0, stream);
   check(cuLaunchCooperativeKernel(f, grid, 1, 1, block, 1, 1, unsigned(smem), stream, args),
@@ -296,11 +306,7 @@ inline void launch_cooperative(
 inline int occupancy(CUkernel kernel, int block, size_t smem)
 {
   CUfunction f = function_of(kernel);
-  if (smem > 48 * 1024)
-  {
-    check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
-          "cuFuncSetAttribute(max dynamic shared memory)");
-  }
+  allow_smem(f, smem);
   int n = 0;
   check(cuOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, block, smem), "cuOccupancyMaxActiveBlocksPerMultiprocessor");
   if (n < 1)
@@ -311,11 +317,10 @@ inline int occupancy(CUkernel kernel, int block, size_t smem)
 }
 
 // Whether the device can run one cluster of `cluster` CTAs of the kernel (sets the kernel's limits).
-inline bool cluster_fits(CUkernel kernel, unsigned cluster, unsigned block, size_t smem)
+inline bool cluster_fits(CUkernel kernel, unsigned cluster, unsigned block, size_t smem, size_t most_smem)
 {
   CUfunction f = function_of(kernel);
-  check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(smem)),
-        "cuFuncSetAttribute(max dynamic shared memory)");
+  allow_smem(f, most_smem);
   check(cuFuncSetAttribute(f, CU_FUNC_ATTRIBUTE_NON_PORTABLE_CLUSTER_SIZE_ALLOWED, 1),
         "cuFuncSetAttribute(non-portable cluster size)");
   CUlaunchAttribute attr{};

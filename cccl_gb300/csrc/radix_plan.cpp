@@ -284,7 +284,8 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
   {
     const int ipt     = int(ceil_div(n, uint64_t(CLUSTER_CTAS) * CLUSTER_TPB));
     const size_t smem = cluster_smem_bytes(kb, vb, ipt);
-    if (cluster_fits(ks.cluster, CLUSTER_CTAS, CLUSTER_TPB, smem))
+    const size_t most = cluster_smem_bytes(kb, vb, cluster_items(kb, vb));
+    if (cluster_fits(ks.cluster, CLUSTER_CTAS, CLUSTER_TPB, smem, most))
     {
       const int result = c.overwrite ? passes & 1 : 1; // the buffer that the passes would end in
       ClusterSortParams p{};
@@ -300,7 +301,7 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
       p.end_bit          = c.end_bit;
       p.codec            = codec;
       p.gate             = c.gate;
-      launch_after("cluster_sort", ks.cluster, CLUSTER_CTAS, CLUSTER_TPB, smem, c.stream, p, true, CLUSTER_CTAS);
+      launch_after("cluster_sort", ks.cluster, CLUSTER_CTAS, CLUSTER_TPB, smem, c.stream, p, true, most, CLUSTER_CTAS);
       *selector = passes & 1;
       return;
     }
@@ -373,7 +374,7 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
       grid        = std::min(grid + levels, sms);
     }
     launch_after("histogram", ks.histogram, grid, unsigned(HISTOGRAM_LANES_TPB), histogram_table_bytes(passes), c.stream, p,
-                 chained);
+                 chained, histogram_table_bytes(MAX_PASSES));
   }
   // 3. one onesweep launch per (pass, portion)
   void* kdst[MAX_PASSES];
