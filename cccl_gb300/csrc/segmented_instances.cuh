@@ -33,7 +33,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::SEG_NETWORK_TPB)                                               \
     gb300_seg_small_k##KB##_v##VB##_##KS(const gb300::SegSortParams p)                                               \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_network_body<KB, KIND, VB, gb300::seg_small_threads(KB, VB), gb300::seg_small_items(KB, VB)>(         \
       p, p.small_list, gb300::SEG_CTR_SMALL, gb300::SEG_CTR_TICKET_SMALL);                                           \
     gb300::chain_end(p.chain);                                                                                       \
@@ -41,7 +41,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::SEG_NETWORK_TPB)                                               \
     gb300_seg_medium_k##KB##_v##VB##_##KS(const gb300::SegSortParams p)                                              \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_network_body<KB, KIND, VB, gb300::seg_medium_threads(KB, VB), gb300::seg_medium_items(KB, VB)>(       \
       p, p.medium_list, gb300::SEG_CTR_MEDIUM, gb300::SEG_CTR_TICKET_MEDIUM);                                        \
     gb300::chain_end(p.chain);                                                                                       \
@@ -56,7 +56,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::seg_block_xs_tpb(KB), gb300::seg_block_xs_minb(KB))            \
     gb300_seg_block_xs_k##KB##_v##VB##_##FS(const gb300::SegSortParams p)                                            \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_block_xs_body<KB, VB, FP, gb300::seg_block_xs_tpb(KB), gb300::seg_block_xs_items(KB),                 \
                              gb300::seg_block_s_bits(KB)>(p);                                                        \
     gb300::chain_end(p.chain);                                                                                       \
@@ -64,7 +64,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::seg_block_s_tpb(KB), gb300::seg_block_s_minb(KB, VB))              \
     gb300_seg_block_s_k##KB##_v##VB##_##FS(const gb300::SegSortParams p)                                             \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_block_s_body<KB, VB, FP, gb300::seg_block_s_tpb(KB), gb300::seg_block_s_items(KB),                    \
                             gb300::seg_block_s_bits(KB)>(p);                                                         \
     gb300::chain_end(p.chain);                                                                                       \
@@ -72,7 +72,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::seg_block_l_tpb(KB), gb300::seg_block_minb(KB))              \
     gb300_seg_block_l_k##KB##_v##VB##_##FS(const gb300::SegSortParams p)                                             \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_block_body<KB, VB, FP, gb300::seg_block_l_tpb(KB), gb300::seg_block_l_items(KB),               \
                           gb300::seg_block_l_bits(KB)>(                                                            \
       p, p.block_l_list, gb300::SEG_CTR_BLOCK_L, gb300::SEG_CTR_TICKET_BLOCK_L);                                     \
@@ -94,7 +94,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::HISTOGRAM_TPB)                                                 \
     gb300_seg_hist_k##KB##_##FS(const gb300::SegDeviceParams p)                                                      \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_device_histogram_body<KB, FP, gb300::HISTOGRAM_TPB>(p);                                               \
     gb300::chain_end(p.chain);                                                                                       \
   }
@@ -104,7 +104,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::SEG_NETWORK_TPB)                                               \
     gb300_seg_small_k##KB##_v##VB##_##KS(const gb300::SegSortParams p)                                               \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_network_body<KB, KIND, VB, gb300::SEG_RSMALL_THREADS, gb300::SEG_RSMALL_ITEMS>(                        \
       p, p.small_list, gb300::SEG_CTR_SMALL, gb300::SEG_CTR_TICKET_SMALL);                                           \
     gb300::chain_end(p.chain);                                                                                       \
@@ -112,7 +112,7 @@ extern "C" __global__ void __launch_bounds__(256) gb300_seg_scan(const gb300::Se
   extern "C" __global__ void __launch_bounds__(gb300::SEG_NETWORK_TPB)                                               \
     gb300_seg_medium_k##KB##_v##VB##_##KS(const gb300::SegSortParams p)                                              \
   {                                                                                                                  \
-    gb300::chain_begin(p.chain);                                                                                     \
+    gb300::chain_begin(p.chain, p.counters + gb300::SEG_CTR_READY);                                                  \
     gb300::seg_network_body<KB, KIND, VB, gb300::SEG_RMEDIUM_THREADS, gb300::SEG_RMEDIUM_ITEMS>(                      \
       p, p.medium_list, gb300::SEG_CTR_MEDIUM, gb300::SEG_CTR_TICKET_MEDIUM);                                        \
     gb300::chain_end(p.chain);                                                                                       \

@@ -102,14 +102,38 @@ __device__ __forceinline__ void wait_for_previous_grid()
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The same for a kernel that may run beside the launches before it, up to the last one with
-// how == CHAIN_WAIT (that one has started, so what it waited for is over): it does its work at once
-// and waits before it ends, so that whoever waits for it has waited for those too.
-__device__ __forceinline__ void chain_begin(int how)
+// The same for a kernel that may run beside the launches before it (how == CHAIN_BESIDE), up to the last
+// one with CHAIN_WAIT: it does its work at once and waits before it ends, so that whoever waits for it
+// has waited for those too.
+//
+// It starts when every CTA of the launch before it has started, and so after the CHAIN_WAIT one has
+// waited; but what that one waited for is visible only to a grid that waits itself. So the CHAIN_WAIT
+// one releases *ready (zeroed earlier in the chain) behind its wait, and the others acquire it, which
+// makes visible all that was visible there: the segment lists, the offsets, the keys. A CTA that
+// does not find it set waits like the first. Called by every thread of the CTA.
+__device__ __forceinline__ void chain_begin(int how, uint32_t* ready)
 {
-  if (how != CHAIN_BESIDE)
+  bool waits = how != CHAIN_BESIDE;
+  if (!waits)
+  {
+    uint32_t set = 0;
+    if (threadIdx.x == 0)
+    {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(set) : "l"(ready) : "memory");
+    }
+    waits = __syncthreads_or(int(set)) == 0;
+  }
+  if (waits)
   {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+  if (how != CHAIN_BESIDE && blockIdx.x == 0)
+  {
+    if (threadIdx.x == 0)
+    {
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(ready), "r"(1u) : "memory");
+    }
+    __syncthreads(); // on its way before the next launch may start
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

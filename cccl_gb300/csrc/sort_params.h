@@ -274,10 +274,11 @@ enum : uint32_t
   SEG_CTR_BLOCK_XS, // block class of the shortest segments (256 threads x 2 keys)
   SEG_CTR_TICKET_BLOCK_XS,
   SEG_CTR_TICKET_PASS0, // one per device pass
+  SEG_CTR_READY = 29,      // set when the kernels before the classes' have ended (chain_begin)
   SEG_CTR_DEVICE_ITEMS = 30, // u64 (two words, 8-byte aligned): keys in device-class segments
   SEG_CTR_WORDS        = 32
 };
-static_assert(SEG_CTR_TICKET_PASS0 + SEG_MAX_PASSES <= SEG_CTR_DEVICE_ITEMS, "segmented counter words overlap");
+static_assert(SEG_CTR_TICKET_PASS0 + SEG_MAX_PASSES <= SEG_CTR_READY, "segmented counter words overlap");
 
 struct DeviceSegment
 {
@@ -319,7 +320,7 @@ struct SegClassifyParams
 
 // How a kernel of a chained launch starts (chain_begin in sort_common.cuh)
 constexpr int CHAIN_WAIT   = 0; // when the launch before it has ended
-constexpr int CHAIN_BESIDE = 1; // at once
+constexpr int CHAIN_BESIDE = 1; // at once, once it has acquired SEG_CTR_READY
 
 struct SegSortParams
 {
