@@ -26,81 +26,99 @@ __device__ __forceinline__ long long load_offset(const void* p, unsigned long lo
   return wide ? static_cast<const long long*>(p)[i] : (long long) static_cast<const int*>(p)[i];
 }
 
-// Compares every element with the one J behind it, then J / 2, ... 1.
-template <class T, int E, int J>
-__device__ __forceinline__ void warp_bitonic_merge(T (&x)[E])
+// Element r of every lane with element r of the lane `mask` away (MIRRORED: with its element E - 1 - r);
+// the lane with `upper` set keeps the larger ones.
+template <bool MIRRORED, class T, int E>
+__device__ __forceinline__ void warp_bitonic_across(T (&x)[E], int mask, bool upper)
 {
-  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int r = 0; r < (MIRRORED ? E / 2 : E); ++r)
+  {
+    const int q = MIRRORED ? E - 1 - r : r;
+    const T a   = __shfl_xor_sync(0xffffffffu, x[q], mask);
+    const T b   = MIRRORED ? __shfl_xor_sync(0xffffffffu, x[r], mask) : a;
+    x[r]        = (x[r] < a) != upper ? x[r] : a;
+    if (MIRRORED)
+    {
+      x[q] = (x[q] < b) != upper ? x[q] : b;
+    }
+  }
+}
+
+template <class T, int E>
+__device__ __forceinline__ void warp_bitonic_exchange(T (&x)[E], int r, int o)
+{
+  const T a = x[r], b = x[o];
+  const bool less = a < b;
+  x[r]            = less ? a : b;
+  x[o]            = less ? b : a;
+}
+
+// Compares every element with the one J behind it in its lane, then J / 2, ... 1.
+template <int J, class T, int E>
+__device__ __forceinline__ void warp_bitonic_inside(T (&x)[E])
+{
 #pragma unroll
   for (int j = J; j >= 1; j /= 2)
   {
-    if (j < E)
-    {
 #pragma unroll
-      for (int r = 0; r < E; ++r)
-      {
-        if ((r & j) == 0)
-        {
-          const T a = x[r], b = x[r | j];
-          const bool less = a < b;
-          x[r]            = less ? a : b;
-          x[r | j]        = less ? b : a;
-        }
-      }
-    }
-    else
+    for (int r = 0; r < E; ++r)
     {
-      const bool upper = (lane & (j / E)) != 0; // keeps the larger one
-#pragma unroll
-      for (int r = 0; r < E; ++r)
+      if ((r & j) == 0)
       {
-        const T a = __shfl_xor_sync(0xffffffffu, x[r], j / E);
-        x[r]      = (x[r] < a) != upper ? x[r] : a;
+        warp_bitonic_exchange(x, r, r | j);
       }
     }
   }
 }
 
-// Sorts blocks of K elements of the warp whose halves are sorted, then of 2 K, ... 32 * E.
-template <class T, int E, int K = 2>
-__device__ __forceinline__ void warp_bitonic_sort(T (&x)[E])
+// Merges the bitonic halves of blocks of 2 * m lanes, m >= 1: elements m lanes apart, then m / 2, ... 1,
+// then inside the lanes.
+template <class T, int E>
+__device__ __forceinline__ void warp_bitonic_merge(T (&x)[E], int m)
 {
   const int lane = threadIdx.x & 31;
-  // element i with element K - 1 - i of its block
+#pragma unroll 1
+  for (; m >= 1; m >>= 1)
+  {
+    warp_bitonic_across<false>(x, m, (lane & m) != 0);
+  }
+  warp_bitonic_inside<E / 2>(x);
+}
+
+// The elements of every lane: blocks of K whose halves are sorted, then of 2 K, ... E.
+template <int K, class T, int E>
+__device__ __forceinline__ void warp_bitonic_lane(T (&x)[E])
+{
   if constexpr (K <= E)
   {
 #pragma unroll
     for (int r = 0; r < E; ++r)
     {
-      const int o = (r & ~(K - 1)) | (K - 1 - (r & (K - 1)));
+      const int o = (r & ~(K - 1)) | (K - 1 - (r & (K - 1))); // element i with element K - 1 - i of its block
       if (r < o)
       {
-        const T a = x[r], b = x[o];
-        const bool less = a < b;
-        x[r]            = less ? a : b;
-        x[o]            = less ? b : a;
+        warp_bitonic_exchange(x, r, o);
       }
     }
+    warp_bitonic_inside<K / 4>(x);
+    warp_bitonic_lane<2 * K>(x);
   }
-  else
+}
+
+// The steps across lanes are loops. Unrolled, the networks are some 70 KB of instructions: a warp with one
+// segment spent its time fetching them (one of 304 i32 keys with i64 values beside 699 of 6000: the call
+// 185 us, 162 so; 155 without that segment), and rows of about 200 i32 keys took 211 us, 191 so.
+template <class T, int E>
+__device__ __forceinline__ void warp_bitonic_sort(T (&x)[E])
+{
+  const int lane = threadIdx.x & 31;
+  warp_bitonic_lane<2>(x);
+#pragma unroll 1
+  for (int m = 1; m < 32; m <<= 1)
   {
-    const bool upper = (lane & (K / E / 2)) != 0;
-#pragma unroll
-    for (int r = 0; r < E / 2; ++r)
-    {
-      const T a    = __shfl_xor_sync(0xffffffffu, x[E - 1 - r], K / E - 1);
-      const T b    = __shfl_xor_sync(0xffffffffu, x[r], K / E - 1);
-      x[r]         = (x[r] < a) != upper ? x[r] : a;
-      x[E - 1 - r] = (x[E - 1 - r] < b) != upper ? x[E - 1 - r] : b;
-    }
-  }
-  if constexpr (K >= 4)
-  {
-    warp_bitonic_merge<T, E, K / 4>(x);
-  }
-  if constexpr (K < 32 * E)
-  {
-    warp_bitonic_sort<T, E, 2 * K>(x);
+    warp_bitonic_across<true>(x, 2 * m - 1, (lane & m) != 0);
+    warp_bitonic_merge(x, m >> 1);
   }
 }
 
@@ -154,7 +172,7 @@ __device__ __forceinline__ void warp_sort_segment(
       const int i = r * 32 + lane;
       x[r]        = i < n ? uint32_t(encode_key<U>(kin[i], codec)) : ~0u;
     }
-    warp_bitonic_sort<uint32_t, E>(x);
+    warp_bitonic_sort(x);
 #pragma unroll
     for (int r = 0; r < E; ++r)
     {
@@ -193,7 +211,7 @@ __device__ __forceinline__ void warp_sort_segment(
         x[r] = T(~T(0)); // above every element: an index has fewer bits than the space below the key
       }
     }
-    warp_bitonic_sort<T, E>(x);
+    warp_bitonic_sort(x);
 #pragma unroll
     for (int r = 0; r < E; ++r)
     {
@@ -273,7 +291,7 @@ __device__ __forceinline__ void group_sort_segment(
     const int i = warp * WE + r * 32 + lane;
     x[r]        = i < n ? uint32_t(encode_key<U>(kin[i], codec)) : ~0u;
   }
-  warp_bitonic_sort<uint32_t, E>(x);
+  warp_bitonic_sort(x);
   // element i of this warp with element i of warp `other`, or (mirrored) with element WE - 1 - i
   auto exchange = [&](int other, bool mirrored) {
 #pragma unroll
@@ -292,10 +310,10 @@ __device__ __forceinline__ void group_sort_segment(
     sync(); // before the next writes
   };
   exchange(warp ^ 1, true);
-  warp_bitonic_merge<uint32_t, E, WE / 2>(x);
+  warp_bitonic_merge(x, 16);
   exchange(warp ^ 3, true);
   exchange(warp ^ 1, false);
-  warp_bitonic_merge<uint32_t, E, WE / 2>(x);
+  warp_bitonic_merge(x, 16);
 #pragma unroll
   for (int r = 0; r < E; ++r)
   {
