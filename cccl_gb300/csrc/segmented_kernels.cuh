@@ -636,7 +636,7 @@ __device__ __forceinline__ void seg_block_s_body(const SegSortParams& p)
   if constexpr (KB == 4 && VB == 0 && FP == FP_NONE)
   {
     static_assert(TPB * ITEMS <= GROUP_SORT_MAX, "the class's longest segment fits a group");
-    static_assert(sizeof(uint32_t) * WARP_SORT_SLOTS * (TPB / 32) <= block_sort_smem(KB, TPB, ITEMS),
+    static_assert(sizeof(uint32_t) * WARP_SORT_SLOTS * (TPB / 32) <= seg_block_smem(KB, TPB, ITEMS),
                   "the groups' exchange fits the class's shared memory");
     if (p.begin_bit == 0 && p.end_bit == 8 * KB)
     {

@@ -677,9 +677,13 @@ GB300_HD constexpr size_t block_merge_smem(int kb, int tpb, int items)
   return round16(size_t(kb) * (size_t(tpb) * items + size_t(tpb) * items / (kb == 8 ? 16 : 32) + 1))
        + round16(size_t(2) * (size_t(tpb) * items + 2 * (size_t(tpb) * items / 64) + 2));
 }
+// A block class's kernel takes the merge sort for whole keys only: under a bit window, and for integer
+// keys alone in the registers of warps (warp_sort.cuh), it needs what the radix form does.
 GB300_HD constexpr size_t seg_block_smem(int kb, int tpb, int items)
 {
-  return seg_block_algo(kb) == SEG_BLOCK_MERGE ? block_merge_smem(kb, tpb, items) : block_sort_smem(kb, tpb, items);
+  const size_t radix = block_sort_smem(kb, tpb, items);
+  const size_t merge = seg_block_algo(kb) == SEG_BLOCK_MERGE ? block_merge_smem(kb, tpb, items) : 0;
+  return radix > merge ? radix : merge;
 }
 } // namespace gb300
 
