@@ -7,7 +7,7 @@
 // a shared-memory sort of every piece, finishes the job. 2^28 u64 keys with u32 values take
 // 2 passes and the finish instead of 8 passes.
 //
-// Whether the top digits split the keys well enough is read off a sample of at most 2^14 keys,
+// Whether the top digits split the keys well enough is read off a sample of at most 2^13 keys,
 // counted inside the histogram kernel (finish_sample); its last CTA picks the route
 // (finish_choose in sort_policy.h) and writes the pass plan: the passes of the digits below
 // the partition are skipped like passes of constant digits. No host synchronisation, so the
@@ -87,7 +87,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   using U                = typename uint_of<KB>::type;
   const int tid          = threadIdx.x;
   const uint32_t samples = p.sample_items; // a multiple of TPB
-  const uint32_t slots   = min(4u * samples, 1u << 14);
+  const uint32_t slots   = finish_sample_slots(samples);
   const int shift        = 8 * KB - 8 * level;
   const U* keys          = static_cast<const U*>(p.keys);
   uint32_t* table        = reinterpret_cast<uint32_t*>(smem);          // [slots]

@@ -334,10 +334,29 @@ GB300_HD constexpr float finish_cost(int kb, int vb)
   return (void) vb, kb == 8 ? 1.1f : 1.4f;
 }
 // Sampled keys: more for larger inputs, whose buckets hold a smaller share of the keys.
+constexpr unsigned FINISH_SAMPLE_FEW  = 4096;
+constexpr unsigned FINISH_SAMPLE_MOST = 8192;
 GB300_HD constexpr unsigned finish_sample_items(unsigned long long n)
 {
-  return n >= (1ull << 24) ? 8192u : 4096u; // a 64 KB table and 8 bytes a key: 128 KB
+  return n >= (1ull << 24) ? FINISH_SAMPLE_MOST : FINISH_SAMPLE_FEW;
 }
+// The sample's hash table has four slots a key, up to 64 KB; table and keys take the place of the
+// histogram's table, which a sort of whole keys launches its CTAs with.
+constexpr unsigned FINISH_SAMPLE_SLOTS = 1u << 14;
+GB300_HD constexpr unsigned finish_sample_slots(unsigned samples)
+{
+  return 4 * samples < FINISH_SAMPLE_SLOTS ? 4 * samples : FINISH_SAMPLE_SLOTS;
+}
+GB300_HD constexpr size_t finish_sample_smem(int kb, unsigned samples)
+{
+  return size_t(4) * finish_sample_slots(samples) + size_t(kb) * samples;
+}
+static_assert(finish_sample_smem(4, FINISH_SAMPLE_MOST) <= histogram_table_bytes(4)
+                && finish_sample_smem(8, FINISH_SAMPLE_MOST) <= histogram_table_bytes(8),
+              "the sample fits the histogram's shared memory");
+static_assert(FINISH_SAMPLE_FEW % HISTOGRAM_LANES_TPB == 0 && FINISH_SAMPLE_MOST % HISTOGRAM_LANES_TPB == 0,
+              "all threads take every round of the sample: it has barriers");
+static_assert(FINISH_SAMPLE_MOST < (1u << 14), "a slot counts in 14 bits");
 
 // Top digits to partition by (0: run every digit pass). `trivial_mask`: passes whose digit is
 // constant; light[l] and heavy[l]: what the sample of S keys found for the top l + 1 digits
