@@ -275,8 +275,11 @@ void radix_sort_dispatch(const RadixPolicy& pol, const RadixKernels& ks, const R
                       reinterpret_cast<uint32_t*>(base + t.lookback_off) + t.lookback_words};
   void* keys_tmp   = base + t.keys_tmp_off;
   void* values_tmp = base + t.values_tmp_off;
-  // buffers that are not 16-byte aligned take every pass (the finish bulk-copies its pieces)
-  const bool finish = t.finish && persistent && ks.finish != nullptr;
+  // buffers that are not 16-byte aligned take every pass (the finish bulk-copies its pieces), and so does
+  // a sort whose output is its input: an even number of passes starts by writing the temporary
+  // buffer, an odd one, which the partition may take, would write the keys it still has to read
+  const bool in_place = c.keys[0] == c.keys[1] || (has_vals && c.values[0] == c.values[1]);
+  const bool finish   = t.finish && persistent && ks.finish != nullptr && !in_place;
   auto* fctrl       = reinterpret_cast<FinishControl*>(base + t.finish_ctrl_off);
 
   // Short sorts: one cluster, one launch. The temporary storage is only used for the status word.

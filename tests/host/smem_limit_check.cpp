@@ -9,98 +9,32 @@
 #include <cstdio>
 #include <map>
 #include <set>
-#include <vector>
 
 #include "abi_common.h"
+
+#include "recording_driver.h"
 
 namespace
 {
 std::map<CUfunction, std::set<int>> limits; // every value set, by function
-std::map<CUfunction, unsigned> most;        // largest launch, by function
 int failures = 0;
+} // namespace
+
+void limit_set(CUfunction f, int bytes)
+{
+  limits[f].insert(bytes);
+}
+
+void role_launched(const char*) {}
 
 void launched(CUfunction f, unsigned smem)
 {
-  most[f] = most[f] > smem ? most[f] : smem;
   if (smem > 48 * 1024 && (limits[f].empty() || smem > unsigned(*limits[f].begin())))
   {
     std::printf("a launch of kernel %p takes %u bytes, a call may set less\n", (void*) f, smem);
     ++failures;
   }
 }
-} // namespace
-
-// ---- the driver ----
-extern "C" {
-CUresult cuGetErrorName(CUresult, const char** s)
-{
-  *s = "error";
-  return CUDA_SUCCESS;
-}
-CUresult cuKernelGetFunction(CUfunction* f, CUkernel k)
-{
-  *f = reinterpret_cast<CUfunction>(k);
-  return CUDA_SUCCESS;
-}
-CUresult cuFuncSetAttribute(CUfunction f, CUfunction_attribute a, int v)
-{
-  if (a == CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES)
-  {
-    limits[f].insert(v);
-  }
-  return CUDA_SUCCESS;
-}
-CUresult cuLaunchKernel(CUfunction f, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned smem,
-                        CUstream, void**, void**)
-{
-  launched(f, smem);
-  return CUDA_SUCCESS;
-}
-CUresult cuLaunchKernelEx(const CUlaunchConfig* c, CUfunction f, void**, void**)
-{
-  launched(f, c->sharedMemBytes);
-  return CUDA_SUCCESS;
-}
-CUresult cuLaunchCooperativeKernel(CUfunction f, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
-                                   unsigned smem, CUstream, void**)
-{
-  launched(f, smem);
-  return CUDA_SUCCESS;
-}
-CUresult cuOccupancyMaxActiveBlocksPerMultiprocessor(int* n, CUfunction, int, size_t)
-{
-  *n = 1;
-  return CUDA_SUCCESS;
-}
-CUresult cuOccupancyMaxActiveClusters(int* n, CUfunction, const CUlaunchConfig*)
-{
-  *n = 1;
-  return CUDA_SUCCESS;
-}
-CUresult cuCtxGetDevice(CUdevice* d)
-{
-  *d = 0;
-  return CUDA_SUCCESS;
-}
-CUresult cuDeviceGetAttribute(int* v, CUdevice_attribute, CUdevice)
-{
-  *v = 152;
-  return CUDA_SUCCESS;
-}
-CUresult cuMemsetD32Async(CUdeviceptr, unsigned, size_t, CUstream)
-{
-  return CUDA_SUCCESS;
-}
-CUresult cuMemcpyAsync(CUdeviceptr, CUdeviceptr, size_t, CUstream)
-{
-  return CUDA_SUCCESS;
-}
-}
-
-namespace gb300
-{
-void notify_launch(const char*, int, CUstream) {}
-} // namespace gb300
 
 int main()
 {
@@ -111,7 +45,6 @@ int main()
     for (int vb : {0, 4, 8})
     {
       limits.clear();
-      most.clear();
       const RadixPolicy pol = make_radix_policy(kb, vb, KIND_UNSIGNED);
       RadixKernels ks{};
       CUkernel* const slots = reinterpret_cast<CUkernel*>(&ks);
