@@ -459,16 +459,16 @@ __device__ __forceinline__ void finish_exchange(uint32_t& a, uint32_t& b)
   a                = x;
 }
 
-// Sorts 32 * PER words in shared memory by one warp (bitonic, PER consecutive words a lane).
+// Sorts c of at most 32 * PER words in shared memory by one warp (bitonic, PER consecutive words a lane).
 template <int PER>
-__device__ __forceinline__ void finish_sort_window(uint32_t* w)
+__device__ __forceinline__ void finish_sort_window(uint32_t* w, int c = 32 * PER)
 {
   const int lane = threadIdx.x & 31;
   uint32_t x[PER];
 #pragma unroll
   for (int k = 0; k < PER; ++k)
   {
-    x[k] = w[lane * PER + k];
+    x[k] = lane * PER + k < c ? w[lane * PER + k] : 0xffffffffu;
   }
 #pragma unroll 1
   for (int size = 2; size <= 32 * PER; size <<= 1)
@@ -507,20 +507,155 @@ __device__ __forceinline__ void finish_sort_window(uint32_t* w)
 #pragma unroll
   for (int k = 0; k < PER; ++k)
   {
-    w[lane * PER + k] = x[k];
+    if (lane * PER + k < c)
+    {
+      w[lane * PER + k] = x[k];
+    }
   }
 }
 
+// Sorts words[0, c) in shared memory by one warp: a bitonic network whose merges start with the mirrored
+// comparison, so that all comparisons point the same way and those with places behind c are left out.
+__device__ __forceinline__ void finish_sort_bin(uint32_t* words, uint32_t c)
+{
+  const uint32_t lane = threadIdx.x & 31;
+  auto compare        = [&](uint32_t i, uint32_t j) {
+    if (j < c)
+    {
+      const uint32_t a = words[i], b = words[j];
+      if (b < a)
+      {
+        words[i] = b;
+        words[j] = a;
+      }
+    }
+  };
+#pragma unroll 1
+  for (uint32_t half = 1; half < c; half <<= 1) // merges sorted blocks of `half` words
+  {
+#pragma unroll 1
+    for (uint32_t t = lane; t < (c + half) / 2u; t += 32) // the pairs behind have a place behind c
+    {
+      const uint32_t o = t & (half - 1u), first = (t - o) * 2u;
+      compare(first + o, first + 2u * half - 1u - o);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t d = half >> 1; d >= 1u; d >>= 1)
+    {
+#pragma unroll 1
+      for (uint32_t t = lane; t < c / 2u; t += 32)
+      {
+        const uint32_t o = t & (d - 1u), first = (t - o) * 2u;
+        compare(first + o, first + o + d);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// The bins of more than FINISH_BIN_MAX words, which the rounds of finish_order would take too long for:
+// each is sorted by the warp whose threads hold its start. Most hold many copies of one key. Returns
+// the keys of the fullest other bin, or 0 where the piece is left to the large form: a warp would
+// have more than FINISH_CROWD_MAX words to sort, or different keys share a place in many words, which
+// one thread would have to put in order. Called by all sorting threads, the words in bin order.
+// 2^26 i64 keys with i32 values, 5 % of the keys 67 times each: 2.21 ms; 5.43 with those pieces left to
+// the large form, 3.48 by all digit passes, 1.46 with keys that differ. Bins of 17 to 64 words stay with
+// the rounds: a network each took 2.73 ms where 30 % of the keys have 20 copies, the rounds 1.97.
+template <int KB, int VB, int FP, bool LARGE>
+__device__ __noinline__ uint32_t
+finish_crowded(const typename uint_of<KB>::type* ks, uint32_t n, const uint16_t* bin16, uint32_t* words, uint32_t* scan_w)
+{
+  using L               = FinishSmem<KB, VB, LARGE>;
+  using U               = typename L::U;
+  constexpr int TPB     = L::TPB;
+  constexpr int NW      = TPB / 32;
+  constexpr int PER     = L::BINS / TPB;
+  constexpr bool DIRECT = L::DIRECT && FP == FP_NONE;
+  const int tid         = threadIdx.x;
+  const int lane        = tid & 31;
+  auto sync             = [] {
+    asm volatile("bar.sync 3, %0;" ::"n"(TPB) : "memory");
+  };
+  auto start_of = [&](int bin) {
+    return bin < L::BINS ? uint32_t(bin16[bin]) : n;
+  };
+  // the fullest of the other bins, and the words that every warp would have to sort
+  uint32_t most = 0, crowd = 0;
+#pragma unroll 1
+  for (int j = 0; j < PER; ++j)
+  {
+    const uint32_t c = start_of(tid * PER + j + 1) - start_of(tid * PER + j);
+    const bool many  = c > uint32_t(FINISH_BIN_MAX);
+    most             = max(most, many ? 0u : c);
+    crowd += many ? c : 0u;
+  }
+  most  = __reduce_max_sync(0xffffffffu, most);
+  crowd = __reduce_add_sync(0xffffffffu, crowd);
+  if (lane == 0)
+  {
+    scan_w[tid >> 5] = most | crowd << 16;
+  }
+  sync();
+  const uint32_t w       = lane < NW ? scan_w[lane] : 0u;
+  const uint32_t fullest = max(__reduce_max_sync(0xffffffffu, w & 0xffffu), 1u);
+  if (__reduce_max_sync(0xffffffffu, w >> 16) > uint32_t(FINISH_CROWD_MAX))
+  {
+    return 0u; // uniform
+  }
+  uint32_t wrong = 0; // neighbours of one place whose keys are out of order
+#pragma unroll 1
+  for (int j = 0; j < PER; ++j)
+  {
+    const uint32_t own   = start_of(tid * PER + j);
+    const uint32_t count = start_of(tid * PER + j + 1) - own;
+    for (uint32_t todo = __ballot_sync(0xffffffffu, count > uint32_t(FINISH_BIN_MAX)); todo != 0u; todo &= todo - 1u)
+    {
+      const int src    = __ffs(todo) - 1;
+      uint32_t* bin    = words + __shfl_sync(0xffffffffu, own, src);
+      const uint32_t c = __shfl_sync(0xffffffffu, count, src);
+      if (c <= 128u)
+      {
+        finish_sort_window<4>(bin, int(c));
+        __syncwarp();
+      }
+      else
+      {
+        finish_sort_bin(bin, c);
+      }
+      if constexpr (!DIRECT)
+      {
+        for (uint32_t i = lane; i + 1u < c; i += 32)
+        {
+          const uint32_t a = bin[i], b = bin[i + 1u];
+          wrong += (a ^ b) <= L::INDEX && digit_source<U, FP>(ks[b & L::INDEX]) < digit_source<U, FP>(ks[a & L::INDEX]);
+        }
+      }
+    }
+  }
+  wrong = __reduce_add_sync(0xffffffffu, wrong);
+  sync(); // scan_w has been read
+  if (lane == 0)
+  {
+    scan_w[tid >> 5] = wrong;
+  }
+  sync(); // the bins are in order
+  const uint32_t all = __reduce_max_sync(0xffffffffu, lane < NW ? scan_w[lane] : 0u);
+  return all <= uint32_t(FINISH_CROWD_WRONG) ? fullest : 0u;
+}
+
 // Orders one piece, the raw keys ks[0, n) (encoded here): words[q] is left with the q-th key's
-// index in its low bits, or the key itself (DIRECT). False, with nothing ordered, when the fullest bin
-// holds more than FINISH_BIN_MAX keys. The bins are zero on entry and used up on return. Called
+// index in its low bits, or the key itself (DIRECT). False, with nothing ordered, when bins hold more
+// keys than finish_crowded takes. The bins are zero on entry and used up on return. Called
 // by all sorting threads. LARGE: the bins follow the knots (finish_knots), for pieces of uneven
 // density, whose keys would crowd into few equal bins.
 //
 // In bin order the words are sorted but for the order inside every bin, so as many
 // rounds of odd-even transposition as the fullest bin has keys sort them. Every thread does
 // its rounds on ITEMS consecutive words in registers (two instructions a pair; one shuffle
-// each way for the pair between two lanes), a warp its stretch of 32 * ITEMS; bins that
+// each way for the pair between two lanes), a warp its stretch of 32 * ITEMS; where a bin needs more
+// than FINISH_ROUNDS_SURE, every warp looks up what its own bins need (above case of 20 copies: 2.09 ms
+// without; a test for order in the loop made sorts of different keys 1 % slower). Bins that
 // straddle two warps' stretches are finished by sorting the 16 or 64 words on either side.
 // Against letting every key count the smaller words of its bin: 2^28 u64 + u32 2.18 -> 1.62 ms.
 template <int KB, int VB, int FP, bool LARGE>
@@ -553,6 +688,12 @@ __device__ __forceinline__ bool finish_order(
   auto order_of = [](U t) {
     return digit_source<U, FP>(t);
   };
+  // bin, then PLACE bits of the place in it (a key outside the range, of a partition that failed, still
+  // gets a bin of the table)
+  [[maybe_unused]] auto place_of = [&](U t, U lo, uint32_t shift, uint32_t scale) {
+    const unsigned long long z = (unsigned long long) uint32_t(U(order_of(t) - lo) >> shift) * scale;
+    return min(uint32_t(z >> (32 - PLACE)), (uint32_t(L::BINS) << PLACE) - 1u);
+  };
 
   // ---- word and arrival place in its bin of every key ----
   uint32_t mine[ITEMS], arrival[ITEMS]; // with keys as words, the bin in arrival's high half
@@ -573,8 +714,6 @@ __device__ __forceinline__ bool finish_order(
           t     = encode_key<U>(t, codec);
           ks[i] = t;
         }
-        // bin, then PLACE bits of the place in it (a key outside the range, of a partition that
-        // failed, still gets a bin of the table)
         uint32_t place;
         if constexpr (LARGE)
         {
@@ -591,8 +730,7 @@ __device__ __forceinline__ bool finish_order(
         }
         else
         {
-          const unsigned long long z = (unsigned long long) uint32_t(U(order_of(t) - lo) >> shift) * scale;
-          place                      = min(uint32_t(z >> (32 - PLACE)), (uint32_t(L::BINS) << PLACE) - 1u);
+          place = place_of(t, lo, shift, scale);
         }
         const uint32_t bin  = place >> PLACE;
         const uint32_t half = (bin & 1u) * 16u;
@@ -664,10 +802,6 @@ __device__ __forceinline__ bool finish_order(
     }
   }
   sync();
-  if (fullest > uint32_t(FINISH_BIN_MAX))
-  {
-    return false; // uniform
-  }
   // ---- the words in bin order ----
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j)
@@ -679,9 +813,41 @@ __device__ __forceinline__ bool finish_order(
     }
   }
   sync();
+  if (fullest > uint32_t(FINISH_BIN_MAX))
+  {
+    fullest = finish_crowded<KB, VB, FP, LARGE>(ks, n, bin16, words, scan_w);
+    if (fullest == 0u)
+    {
+      return false; // uniform
+    }
+  }
   // ---- sorted inside every bin ----
+  uint32_t rounds       = fullest;
   const uint32_t first  = uint32_t(tid) * ITEMS; // this thread's words
   const bool warp_works = uint32_t(warp) * (32 * ITEMS) < n;
+  if (fullest > uint32_t(FINISH_ROUNDS_SURE) && warp_works)
+  {
+    // few warps hold a piece's fullest bins: the fullest of this warp's
+    auto bin_of = [&](uint32_t q) {
+      if constexpr (DIRECT)
+      {
+        return place_of(U(words[q]), U(piece->lo), piece->shift, piece->scale) >> PLACE;
+      }
+      else
+      {
+        return words[q] >> (L::INDEX_BITS + PLACE);
+      }
+    };
+    const uint32_t last = bin_of(min(uint32_t(warp + 1) * (32 * ITEMS), n) - 1u);
+    uint32_t own        = 0;
+#pragma unroll 1
+    for (uint32_t b = bin_of(uint32_t(warp) * (32 * ITEMS)) + lane; b <= last; b += 32)
+    {
+      const uint32_t c = (b + 1u < uint32_t(L::BINS) ? uint32_t(bin16[b + 1u]) : n) - bin16[b];
+      own              = max(own, c > uint32_t(FINISH_BIN_MAX) ? 0u : c);
+    }
+    rounds = __reduce_max_sync(0xffffffffu, own);
+  }
   if (warp_works)
   {
     uint32_t v[ITEMS];
@@ -703,7 +869,7 @@ __device__ __forceinline__ bool finish_order(
         v[k] = first + k < n ? v[k] : 0xffffffffu; // behind the piece: stays behind
       }
     }
-    for (uint32_t r = 0; r < fullest; r += 2)
+    for (uint32_t r = 0; r < rounds; r += 2)
     {
 #pragma unroll
       for (int k = 0; k + 1 < ITEMS; k += 2)
@@ -781,17 +947,22 @@ __device__ __forceinline__ bool finish_order(
         {
           ++end;
         }
-        // insertion sort of words[from, end)
+        // insertion sort of words[from, end), by index among equal keys: they are in that order
+        U largest = order_of(ks[words[from] & L::INDEX]);
         for (uint32_t r = from + 1u; r < end; ++r)
         {
           const uint32_t w = words[r];
           const U t        = order_of(ks[w & L::INDEX]);
-          uint32_t q       = r;
+          if (!(t < largest))
+          {
+            largest = t; // of copies of one key, all the others
+            continue;
+          }
+          uint32_t q = r;
           while (q > from)
           {
             const uint32_t o = words[q - 1u];
-            const U to       = order_of(ks[o & L::INDEX]);
-            if (to < t || (to == t && o < w))
+            if (!(t < order_of(ks[o & L::INDEX])))
             {
               break;
             }
