@@ -150,7 +150,7 @@ struct HistogramParams
   int hist_ctas;              // CTAs that count keys (0: all); the last sample_levels CTAs sample
   FinishControl* finish;      // null: every digit pass runs
   int sample_levels;
-  uint32_t sample_items;      // keys sampled: 2^12 or 2^13
+  uint32_t sample_items;      // keys sampled: 2^11 to 2^13
   uint32_t sample_heavy;      // sampled keys of one prefix that make its bucket too large
   uint32_t sample_heavy_first; // the same for the first 2^10 sampled keys alone
   uint32_t finish_cap;        // largest piece the finish's first launch takes

@@ -323,9 +323,10 @@ GB300_HD constexpr size_t finish_smem_bytes(int kb, int vb, bool large)
   return round16(kb * cap) + 16 + (vb > 0 ? round16(vb * cap) + 16 : 0) + size_t(2) * finish_bins(kb, vb, large)
        + round16(4 * cap) + (large ? size_t(24) * FINISH_KNOTS : 0) + 512;
 }
-// Smallest sort that takes the sample and, if it promises enough, the partition-and-finish route:
-// below, the sample and two launches (17 us at 2^22 items) weigh too much where it is not taken.
-// Four-byte keys gain less (2 passes of 4).
+// Smallest sort that takes the sample and, if it promises enough, the partition-and-finish route. Where it
+// does not, the sample and two launches that return are lost: u64 keys with u32 values, ANDs of
+// three words, 297 us -> 300 at 2^22 items, 522 -> 529 at 2^23, 939 -> 943 at 2^24; taken, with uniform
+// keys, 298 -> 170, 524 -> 261, 950 -> 438. Four-byte keys gain less (2 passes of 4).
 GB300_HD constexpr unsigned long long finish_min_items(int kb)
 {
   return kb == 8 ? 1ull << 22 : 1ull << 26;
@@ -336,12 +337,14 @@ GB300_HD constexpr float finish_cost(int kb, int vb)
 {
   return (void) vb, kb == 8 ? 1.1f : 1.4f;
 }
-// Sampled keys: more for larger inputs, whose buckets hold a smaller share of the keys.
-constexpr unsigned FINISH_SAMPLE_FEW  = 4096;
+// Sampled keys: more for larger inputs, whose buckets hold a smaller share of the keys. A pair of them stands
+// for as many keys at 2^22 items and 2048 as at 2^26 and 8192; below 2^23 the sample takes longer than
+// the count beside it (4096 at 2^22: 303 us where 2048 take 300, all passes 297).
+constexpr unsigned FINISH_SAMPLE_FEW  = 2048;
 constexpr unsigned FINISH_SAMPLE_MOST = 8192;
 GB300_HD constexpr unsigned finish_sample_items(unsigned long long n)
 {
-  return n >= (1ull << 24) ? FINISH_SAMPLE_MOST : FINISH_SAMPLE_FEW;
+  return n >= (1ull << 24) ? FINISH_SAMPLE_MOST : n >= (1ull << 23) ? 2 * FINISH_SAMPLE_FEW : FINISH_SAMPLE_FEW;
 }
 // The sample's hash table has four slots a key, up to 64 KB; table and keys take the place of the
 // histogram's table, which a sort of whole keys launches its CTAs with.
