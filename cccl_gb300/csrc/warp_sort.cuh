@@ -14,8 +14,8 @@
 //
 // What bounds it: instruction issue, 2 to 3 instructions a slot and lane for the keys themselves, no
 // barrier of the CTA and no pass over shared memory but the transposition in front of the
-// coalesced stores. Sixteen million i32 keys in rows of about 200: 106 us, 442 with one CTA and four
-// digit passes a segment; the class's share of 2^27 f32+i32 in uneven segments: 86 us, was 116.
+// coalesced stores. Sixteen million i32 keys in rows of about 200: 82 us, 442 with one CTA and four
+// digit passes a segment; the class's share of 2^27 f32+i32 in uneven segments: 64 us, was 116.
 #pragma once
 
 #include "radix_kernels.cuh"
