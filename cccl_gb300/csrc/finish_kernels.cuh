@@ -341,6 +341,7 @@ struct FinishSmem
   // low bits of a word: the item's index in the piece; the others are its place in the key range
   static constexpr int INDEX_BITS = LARGE ? 14 : 13;
   static constexpr uint32_t INDEX = (1u << INDEX_BITS) - 1u;
+  static constexpr int PLACE_BITS = 32 - INDEX_BITS - 13; // of the place in the bin: a word is bin, place, index
   // four-byte integer keys without values: equal keys cannot be told apart, the words are the
   // keys (not so floating-point keys, whose zeros are equal but differ)
   static constexpr bool DIRECT = KB == 4 && VB == 0 && !LARGE;
@@ -516,14 +517,15 @@ __device__ __forceinline__ void finish_sort_window(uint32_t* w, int c = 32 * PER
 
 // Sorts words[0, c) in shared memory by one warp: a bitonic network whose merges start with the mirrored
 // comparison, so that all comparisons point the same way and those with places behind c are left out.
-__device__ __forceinline__ void finish_sort_bin(uint32_t* words, uint32_t c)
+template <class Less>
+__device__ __forceinline__ void finish_sort_words(uint32_t* words, uint32_t c, Less&& less)
 {
   const uint32_t lane = threadIdx.x & 31;
   auto compare        = [&](uint32_t i, uint32_t j) {
     if (j < c)
     {
       const uint32_t a = words[i], b = words[j];
-      if (b < a)
+      if (less(b, a))
       {
         words[i] = b;
         words[j] = a;
@@ -554,56 +556,187 @@ __device__ __forceinline__ void finish_sort_bin(uint32_t* words, uint32_t c)
   }
 }
 
+// Bit k: a run of words of one place has its second word at place k of this thread's.
+template <class L>
+__device__ __forceinline__ uint32_t finish_tie_starts(uint32_t n, const uint32_t* words)
+{
+  const uint32_t first  = threadIdx.x * L::ITEMS;
+  uint32_t ties         = 0; // bit k: the thread's k-th word is like the one before it
+  const uint4* group    = reinterpret_cast<const uint4*>(words + first);
+  const uint32_t before = first > 0u ? words[first - 1u] : ~words[0];
+  uint32_t last         = before;
+#pragma unroll
+  for (int g = 0; g < L::ITEMS / 4; ++g)
+  {
+    const uint4 x = group[g];
+    ties |= (last ^ x.x) <= L::INDEX ? 1u << (4 * g) : 0u;
+    ties |= (x.x ^ x.y) <= L::INDEX ? 2u << (4 * g) : 0u;
+    ties |= (x.y ^ x.z) <= L::INDEX ? 4u << (4 * g) : 0u;
+    ties |= (x.z ^ x.w) <= L::INDEX ? 8u << (4 * g) : 0u;
+    last = x.w;
+  }
+  if (first + L::ITEMS > n)
+  {
+    ties &= (1u << (n > first ? n - first : 0u)) - 1u;
+  }
+  const bool joined = (ties & 1u) != 0u && first > 1u && (words[first - 2u] ^ before) <= L::INDEX;
+  return ties & ~(ties << 1) & (joined ? ~1u : ~0u);
+}
+
+// End of the run that starts at `from`, if it has FINISH_RUN_MAX words at most; else a place behind those.
+template <class L>
+__device__ __forceinline__ uint32_t finish_tie_end(uint32_t n, const uint32_t* words, uint32_t from)
+{
+  uint32_t end = from + 2u;
+  while (end < n && end - from <= uint32_t(FINISH_RUN_MAX) && (words[end] ^ words[from]) <= L::INDEX)
+  {
+    ++end;
+  }
+  return end;
+}
+
+// Insertion sort of words[from, end), a run, by one thread: by index among equal keys, as which they come.
+template <class L, int FP>
+__device__ __forceinline__ void finish_insert(const typename L::U* ks, uint32_t* words, uint32_t from, uint32_t end)
+{
+  using U  = typename L::U;
+  auto key = [&](uint32_t w) {
+    return digit_source<U, FP>(ks[w & L::INDEX]);
+  };
+  U largest = key(words[from]);
+  for (uint32_t r = from + 1u; r < end; ++r)
+  {
+    const uint32_t w = words[r];
+    const U t        = key(w);
+    if (!(t < largest))
+    {
+      largest = t; // of copies of one key, all the others
+      continue;
+    }
+    uint32_t q = r;
+    uint32_t o = words[r - 1u]; // the largest one's
+    do
+    {
+      words[q] = o;
+      --q;
+      o = q > from ? words[q - 1u] : w;
+    } while (t < key(o));
+    words[q] = w;
+  }
+}
+
+// Orders a run of words of one place, more than FINISH_RUN_MAX of at most `most`, by their keys, and by
+// index among equal ones, as which they come. By one warp: mostly they are copies of a key, in order.
+template <int KB, int VB, int FP, bool LARGE>
+__device__ __forceinline__ void finish_run(const typename uint_of<KB>::type* ks, uint32_t* run, uint32_t most)
+{
+  using L             = FinishSmem<KB, VB, LARGE>;
+  const uint32_t lane = threadIdx.x & 31;
+  auto key            = [&](uint32_t w) {
+    return digit_source<typename L::U, FP>(ks[w & L::INDEX]);
+  };
+  const uint32_t place = run[0];
+  uint32_t c           = 0;
+  uint32_t other       = 0;
+  while (other == 0u)
+  {
+    const uint32_t i = c + lane;
+    other            = __ballot_sync(0xffffffffu, i >= most || (run[i] ^ place) > L::INDEX);
+    c += other != 0u ? uint32_t(__ffs(other)) - 1u : 32u;
+  }
+  bool wrong = false;
+  for (uint32_t i = lane; i + 1u < c; i += 32)
+  {
+    wrong |= key(run[i + 1u]) < key(run[i]);
+  }
+  if (!__any_sync(0xffffffffu, wrong))
+  {
+    return;
+  }
+  finish_sort_words(run, c, [&](uint32_t x, uint32_t y) {
+    const auto kx = key(x), ky = key(y);
+    return kx < ky || (kx == ky && x < y);
+  });
+}
+
+// The runs of words of one place: the whole keys decide, the index among equal ones. One thread a run; a
+// warp the long ones, which only pieces with bins above FINISH_RUN_MAX (`deep`) hold. A function of its
+// own for the registers of what is around it: inline, sorts of different keys took 1 % longer. 4.4 M u64
+// keys, 5 % in clusters of 25 that differ in their low 21 bits: 222 us; 284 with every run by one
+// thread, 257 by all digit passes. Called by all sorting threads, which have to wait for each other behind it.
+template <int KB, int VB, int FP, bool LARGE>
+__device__ __noinline__ void
+finish_ties(const typename uint_of<KB>::type* ks, uint32_t n, uint32_t* words, bool deep)
+{
+  using L = FinishSmem<KB, VB, LARGE>;
+  static_assert(L::ITEMS <= FINISH_RUN_MAX + 1, "at most one long run has its second word in a thread");
+  const uint32_t first = threadIdx.x * L::ITEMS;
+  uint32_t starts      = first < n ? finish_tie_starts<L>(n, words) : 0u;
+  asm volatile("bar.sync 3, %0;" ::"n"(L::TPB) : "memory");
+  uint32_t long_run = 0xffffffffu;
+  while (starts != 0u)
+  {
+    const uint32_t from = first + uint32_t(__ffs(starts)) - 2u;
+    starts &= starts - 1u;
+    const uint32_t end = finish_tie_end<L>(n, words, from);
+    if (end - from > uint32_t(FINISH_RUN_MAX))
+    {
+      long_run = from;
+    }
+    else
+    {
+      finish_insert<L, FP>(ks, words, from, end);
+    }
+  }
+  if (deep)
+  {
+    for (uint32_t todo = __ballot_sync(0xffffffffu, long_run != 0xffffffffu); todo != 0u; todo &= todo - 1u)
+    {
+      const uint32_t from = __shfl_sync(0xffffffffu, long_run, __ffs(todo) - 1);
+      finish_run<KB, VB, FP, LARGE>(ks, words + from, n - from);
+    }
+  }
+}
+
 // The bins of more than FINISH_BIN_MAX words, which the rounds of finish_order would take too long for:
-// each is sorted by the warp whose threads hold its start. Most hold many copies of one key. Returns
-// the keys of the fullest other bin, or 0 where the piece is left to the large form: a warp would
-// have more than FINISH_CROWD_MAX words to sort, or different keys share a place in many words, which
-// one thread would have to put in order. Called by all sorting threads, the words in bin order.
-// 2^26 i64 keys with i32 values, 5 % of the keys 67 times each: 2.21 ms; 5.43 with those pieces left to
+// each is sorted by the warp whose threads hold its start. Most hold many copies of one key. False, with
+// nothing sorted, where a warp would have more than FINISH_CROWD_MAX words to sort: the piece is left to
+// the large form. Called by all sorting threads, the words in bin order.
+// 2^26 i64 keys with i32 values, 5 % of the keys 67 times each: 1.87 ms; 5.43 with those pieces left to
 // the large form, 3.48 by all digit passes, 1.46 with keys that differ. Bins of 17 to 64 words stay with
 // the rounds: a network each took 2.73 ms where 30 % of the keys have 20 copies, the rounds 1.97.
-template <int KB, int VB, int FP, bool LARGE>
-__device__ __noinline__ uint32_t
-finish_crowded(const typename uint_of<KB>::type* ks, uint32_t n, const uint16_t* bin16, uint32_t* words, uint32_t* scan_w)
+template <int KB, int VB, bool LARGE>
+__device__ __noinline__ bool finish_crowded(uint32_t n, const uint16_t* bin16, uint32_t* words, uint32_t* scan_w)
 {
-  using L               = FinishSmem<KB, VB, LARGE>;
-  using U               = typename L::U;
-  constexpr int TPB     = L::TPB;
-  constexpr int NW      = TPB / 32;
-  constexpr int PER     = L::BINS / TPB;
-  constexpr bool DIRECT = L::DIRECT && FP == FP_NONE;
-  const int tid         = threadIdx.x;
-  const int lane        = tid & 31;
-  auto sync             = [] {
+  using L           = FinishSmem<KB, VB, LARGE>;
+  constexpr int TPB = L::TPB;
+  constexpr int NW  = TPB / 32;
+  constexpr int PER = L::BINS / TPB;
+  const int tid     = threadIdx.x;
+  const int lane    = tid & 31;
+  auto sync         = [] {
     asm volatile("bar.sync 3, %0;" ::"n"(TPB) : "memory");
   };
   auto start_of = [&](int bin) {
     return bin < L::BINS ? uint32_t(bin16[bin]) : n;
   };
-  // the fullest of the other bins, and the words that every warp would have to sort
-  uint32_t most = 0, crowd = 0;
+  uint32_t crowd = 0; // words that this warp would have to sort
 #pragma unroll 1
   for (int j = 0; j < PER; ++j)
   {
     const uint32_t c = start_of(tid * PER + j + 1) - start_of(tid * PER + j);
-    const bool many  = c > uint32_t(FINISH_BIN_MAX);
-    most             = max(most, many ? 0u : c);
-    crowd += many ? c : 0u;
+    crowd += c > uint32_t(FINISH_BIN_MAX) ? c : 0u;
   }
-  most  = __reduce_max_sync(0xffffffffu, most);
   crowd = __reduce_add_sync(0xffffffffu, crowd);
   if (lane == 0)
   {
-    scan_w[tid >> 5] = most | crowd << 16;
+    scan_w[tid >> 5] = crowd;
   }
   sync();
-  const uint32_t w       = lane < NW ? scan_w[lane] : 0u;
-  const uint32_t fullest = max(__reduce_max_sync(0xffffffffu, w & 0xffffu), 1u);
-  if (__reduce_max_sync(0xffffffffu, w >> 16) > uint32_t(FINISH_CROWD_MAX))
+  if (__reduce_max_sync(0xffffffffu, lane < NW ? scan_w[lane] : 0u) > uint32_t(FINISH_CROWD_MAX))
   {
-    return 0u; // uniform
+    return false; // uniform
   }
-  uint32_t wrong = 0; // neighbours of one place whose keys are out of order
 #pragma unroll 1
   for (int j = 0; j < PER; ++j)
   {
@@ -617,31 +750,57 @@ finish_crowded(const typename uint_of<KB>::type* ks, uint32_t n, const uint16_t*
       if (c <= 128u)
       {
         finish_sort_window<4>(bin, int(c));
-        __syncwarp();
       }
       else
       {
-        finish_sort_bin(bin, c);
-      }
-      if constexpr (!DIRECT)
-      {
-        for (uint32_t i = lane; i + 1u < c; i += 32)
-        {
-          const uint32_t a = bin[i], b = bin[i + 1u];
-          wrong += (a ^ b) <= L::INDEX && digit_source<U, FP>(ks[b & L::INDEX]) < digit_source<U, FP>(ks[a & L::INDEX]);
-        }
+        finish_sort_words(bin, c, [](uint32_t x, uint32_t y) {
+          return x < y;
+        });
       }
     }
   }
-  wrong = __reduce_add_sync(0xffffffffu, wrong);
-  sync(); // scan_w has been read
-  if (lane == 0)
-  {
-    scan_w[tid >> 5] = wrong;
-  }
   sync(); // the bins are in order
-  const uint32_t all = __reduce_max_sync(0xffffffffu, lane < NW ? scan_w[lane] : 0u);
-  return all <= uint32_t(FINISH_CROWD_WRONG) ? fullest : 0u;
+  return true;
+}
+
+// Bin, then PLACE_BITS bits of the place in it, of a key `above` the piece's lowest (a key outside the range, of
+// a partition that failed, still gets a bin of the table).
+template <class L>
+__device__ __forceinline__ uint32_t finish_place(typename L::U above, uint32_t shift, uint32_t scale)
+{
+  const unsigned long long z = (unsigned long long) uint32_t(above >> shift) * scale;
+  return min(uint32_t(z >> (32 - L::PLACE_BITS)), (uint32_t(L::BINS) << L::PLACE_BITS) - 1u);
+}
+
+// Rounds that a warp's own words need: the keys of the fullest bin among theirs that the rounds sort. Few
+// warps hold a piece's fullest bins. Called by whole warps that have words, these in bin order.
+template <int KB, int VB, int FP, bool LARGE>
+__device__ __noinline__ uint32_t
+finish_rounds(const FinishPiece* piece, uint32_t n, const uint16_t* bin16, const uint32_t* words)
+{
+  using L               = FinishSmem<KB, VB, LARGE>;
+  using U               = typename L::U;
+  constexpr bool DIRECT = L::DIRECT && FP == FP_NONE;
+  const uint32_t first  = (threadIdx.x >> 5) * (32 * L::ITEMS);
+  auto bin_of           = [&](uint32_t q) {
+    if constexpr (DIRECT)
+    {
+      return finish_place<L>(U(U(words[q]) - U(piece->lo)), piece->shift, piece->scale) >> L::PLACE_BITS;
+    }
+    else
+    {
+      return words[q] >> (L::INDEX_BITS + L::PLACE_BITS);
+    }
+  };
+  const uint32_t last = bin_of(min(first + 32u * L::ITEMS, n) - 1u);
+  uint32_t own        = 0;
+#pragma unroll 1
+  for (uint32_t b = bin_of(first) + (threadIdx.x & 31); b <= last; b += 32)
+  {
+    const uint32_t c = (b + 1u < uint32_t(L::BINS) ? uint32_t(bin16[b + 1u]) : n) - bin16[b];
+    own              = max(own, c > uint32_t(FINISH_BIN_MAX) ? 0u : c);
+  }
+  return __reduce_max_sync(0xffffffffu, own);
 }
 
 // Orders one piece, the raw keys ks[0, n) (encoded here): words[q] is left with the q-th key's
@@ -675,7 +834,7 @@ __device__ __forceinline__ bool finish_order(
   constexpr int ITEMS   = L::ITEMS;
   constexpr int NW      = TPB / 32;
   constexpr bool DIRECT = L::DIRECT && FP == FP_NONE;
-  constexpr int PLACE   = 32 - L::INDEX_BITS - 13; // bits of the place in the bin: a word is bin, place, index
+  constexpr int PLACE   = L::PLACE_BITS;
   static_assert(ITEMS % 4 == 0 && ITEMS * 32 >= 64, "16-byte groups; the windows between warps do not overlap");
   static_assert(FINISH_BIN_MAX <= 64 && ITEMS * 32 >= 128, "a bin across two stretches lies in its window");
   const uint16_t* bin16 = reinterpret_cast<const uint16_t*>(bins);
@@ -687,12 +846,6 @@ __device__ __forceinline__ bool finish_order(
   };
   auto order_of = [](U t) {
     return digit_source<U, FP>(t);
-  };
-  // bin, then PLACE bits of the place in it (a key outside the range, of a partition that failed, still
-  // gets a bin of the table)
-  [[maybe_unused]] auto place_of = [&](U t, U lo, uint32_t shift, uint32_t scale) {
-    const unsigned long long z = (unsigned long long) uint32_t(U(order_of(t) - lo) >> shift) * scale;
-    return min(uint32_t(z >> (32 - PLACE)), (uint32_t(L::BINS) << PLACE) - 1u);
   };
 
   // ---- word and arrival place in its bin of every key ----
@@ -730,7 +883,7 @@ __device__ __forceinline__ bool finish_order(
         }
         else
         {
-          place = place_of(t, lo, shift, scale);
+          place = finish_place<L>(U(order_of(t) - lo), shift, scale);
         }
         const uint32_t bin  = place >> PLACE;
         const uint32_t half = (bin & 1u) * 16u;
@@ -813,13 +966,9 @@ __device__ __forceinline__ bool finish_order(
     }
   }
   sync();
-  if (fullest > uint32_t(FINISH_BIN_MAX))
+  if (fullest > uint32_t(FINISH_BIN_MAX) && !finish_crowded<KB, VB, LARGE>(n, bin16, words, scan_w))
   {
-    fullest = finish_crowded<KB, VB, FP, LARGE>(ks, n, bin16, words, scan_w);
-    if (fullest == 0u)
-    {
-      return false; // uniform
-    }
+    return false; // uniform
   }
   // ---- sorted inside every bin ----
   uint32_t rounds       = fullest;
@@ -827,26 +976,7 @@ __device__ __forceinline__ bool finish_order(
   const bool warp_works = uint32_t(warp) * (32 * ITEMS) < n;
   if (fullest > uint32_t(FINISH_ROUNDS_SURE) && warp_works)
   {
-    // few warps hold a piece's fullest bins: the fullest of this warp's
-    auto bin_of = [&](uint32_t q) {
-      if constexpr (DIRECT)
-      {
-        return place_of(U(words[q]), U(piece->lo), piece->shift, piece->scale) >> PLACE;
-      }
-      else
-      {
-        return words[q] >> (L::INDEX_BITS + PLACE);
-      }
-    };
-    const uint32_t last = bin_of(min(uint32_t(warp + 1) * (32 * ITEMS), n) - 1u);
-    uint32_t own        = 0;
-#pragma unroll 1
-    for (uint32_t b = bin_of(uint32_t(warp) * (32 * ITEMS)) + lane; b <= last; b += 32)
-    {
-      const uint32_t c = (b + 1u < uint32_t(L::BINS) ? uint32_t(bin16[b + 1u]) : n) - bin16[b];
-      own              = max(own, c > uint32_t(FINISH_BIN_MAX) ? 0u : c);
-    }
-    rounds = __reduce_max_sync(0xffffffffu, own);
+    rounds = finish_rounds<KB, VB, FP, LARGE>(piece, n, bin16, words);
   }
   if (warp_works)
   {
@@ -909,70 +1039,7 @@ __device__ __forceinline__ bool finish_order(
   sync();
   if (!DIRECT && (LARGE || piece->exact == 0u))
   {
-    // ---- runs of words of the same place: the whole keys decide, the index among equal ones ----
-    uint32_t starts = 0; // bit k: a run's second word is this thread's k-th
-    if (warp_works)
-    {
-      uint32_t ties      = 0; // bit k: the thread's k-th word is like the one before it
-      const uint4* group = reinterpret_cast<const uint4*>(words + first);
-      const uint32_t before = first > 0u ? words[first - 1u] : ~words[0];
-      uint32_t last         = before;
-#pragma unroll
-      for (int g = 0; g < ITEMS / 4; ++g)
-      {
-        const uint4 x = group[g];
-        ties |= (last ^ x.x) <= L::INDEX ? 1u << (4 * g) : 0u;
-        ties |= (x.x ^ x.y) <= L::INDEX ? 2u << (4 * g) : 0u;
-        ties |= (x.y ^ x.z) <= L::INDEX ? 4u << (4 * g) : 0u;
-        ties |= (x.z ^ x.w) <= L::INDEX ? 8u << (4 * g) : 0u;
-        last = x.w;
-      }
-      if (first + ITEMS > n)
-      {
-        ties &= (1u << (n > first ? n - first : 0u)) - 1u;
-      }
-      // a run belongs to the thread in which its second word lies
-      const bool joined = (ties & 1u) != 0u && first > 1u && (words[first - 2u] ^ before) <= L::INDEX;
-      starts            = ties & ~(ties << 1) & (joined ? ~1u : ~0u);
-    }
-    sync();
-    {
-      while (starts != 0u)
-      {
-        const uint32_t k = uint32_t(__ffs(starts)) - 1u;
-        starts &= starts - 1u;
-        const uint32_t from = first + k - 1u;
-        uint32_t end        = from + 2u;
-        while (end < n && (words[end] ^ words[from]) <= L::INDEX)
-        {
-          ++end;
-        }
-        // insertion sort of words[from, end), by index among equal keys: they are in that order
-        U largest = order_of(ks[words[from] & L::INDEX]);
-        for (uint32_t r = from + 1u; r < end; ++r)
-        {
-          const uint32_t w = words[r];
-          const U t        = order_of(ks[w & L::INDEX]);
-          if (!(t < largest))
-          {
-            largest = t; // of copies of one key, all the others
-            continue;
-          }
-          uint32_t q = r;
-          while (q > from)
-          {
-            const uint32_t o = words[q - 1u];
-            if (!(t < order_of(ks[o & L::INDEX])))
-            {
-              break;
-            }
-            words[q] = o;
-            --q;
-          }
-          words[q] = w;
-        }
-      }
-    }
+    finish_ties<KB, VB, FP, LARGE>(ks, n, words, fullest > uint32_t(FINISH_RUN_MAX));
     sync();
   }
   return true;

@@ -242,9 +242,9 @@ GB300_HD inline void plan_pass_words(uint32_t* plan, int num_passes, int plan_mo
 
 // ---- partition and finish (finish_kernels.cuh) ----
 constexpr int FINISH_BIN_MAX        = 64;      // keys of a bin that the rounds of the finish take
-constexpr int FINISH_ROUNDS_SURE    = 12;      // more rounds: every warp takes those that its own bins need
+constexpr int FINISH_ROUNDS_SURE    = 16;      // more rounds: every warp takes those that its own bins need
 constexpr int FINISH_CROWD_MAX      = 512;     // keys of larger bins that a warp of the finish takes
-constexpr int FINISH_CROWD_WRONG    = 2;       // neighbours among them that it leaves to one thread
+constexpr int FINISH_RUN_MAX        = 23;      // words of one place that one thread orders; longer runs are a warp's
 constexpr int FINISH_KNOTS          = 32;      // stretches of a large piece's bins
 constexpr int FINISH_SMALLEST_PIECE = 2;       // piece_items is at least CAP / 2
 constexpr int FINISH_REST_ITEMS     = 4;

@@ -48,7 +48,7 @@ def _groups(case, rng):
 @pytest.mark.parametrize(
     "case,large",
     [("copies64", False), ("copies65", False), ("copies128", False), ("copies129", False), ("copies300", False),
-     ("copies512", None), ("copies513", True), ("copies700", True), ("a_few_others", None), ("many_others", True),
+     ("copies512", None), ("copies513", True), ("copies700", True), ("a_few_others", None), ("many_others", False),
      ("side_by_side", None)],
 )
 def test_eight_byte_keys(oracle, case, large):
