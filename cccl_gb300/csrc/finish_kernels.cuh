@@ -57,14 +57,16 @@ __device__ __noinline__ uint32_t finish_digits(const HistogramParams& p, uint32_
 {
   const FinishControl* f = p.finish;
   unsigned long long light[8];
-  uint32_t heavy[8];
+  uint32_t heavy[8], partners[8], paired[8];
   for (int l = 0; l < KB; ++l)
   {
-    light[l] = __ldcg(&f->light[l]);
-    heavy[l] = __ldcg(&f->heavy[l]);
+    light[l]    = __ldcg(&f->light[l]);
+    heavy[l]    = __ldcg(&f->heavy[l]);
+    partners[l] = __ldcg(&f->partners[l]);
+    paired[l]   = __ldcg(&f->paired[l]);
   }
   return uint32_t(finish_choose(KB, trivial_mask, light, heavy, p.num_items, p.sample_items, p.finish_cap, p.finish_cost,
-                                p.plan_mode, piece));
+                                p.plan_mode, piece, partners, paired));
 }
 
 // A level is sampled: the thread that counts the last one makes the choice for no trivial digit.
@@ -92,7 +94,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   const U* keys          = static_cast<const U*>(p.keys);
   uint32_t* table        = reinterpret_cast<uint32_t*>(smem);          // [slots]
   U* sampled             = reinterpret_cast<U*>(smem + 4 * size_t(slots)); // [samples], later every key's slot
-  __shared__ uint32_t light_sum, heavy_sum;
+  __shared__ uint32_t light_sum, heavy_sum, partners_sum, paired_sum;
   const uint32_t n = uint32_t(p.num_items); // below 2^31
   const int half   = finish_sample_half(n);
 #pragma unroll 1
@@ -108,8 +110,10 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   }
   if (tid == 0)
   {
-    light_sum = 0u;
-    heavy_sum = 0u;
+    light_sum    = 0u;
+    heavy_sum    = 0u;
+    partners_sum = 0u;
+    paired_sum   = 0u;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
@@ -178,6 +182,7 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   __syncthreads();
   uint32_t light = 0u; // groups below the limit: their sum fits
   uint32_t heavy = 0u;
+  uint32_t partners = 0u, paired = 0u; // sum of (size - 1) over all keys, and keys in groups of 2 to 4
 #pragma unroll 1
   for (uint32_t i = tid; i < samples; i += TPB)
   {
@@ -189,9 +194,13 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
     const bool few = c < (level == KB ? min(limit, 4u) : limit);
     light += few ? c - 1u : 0u;
     heavy += level == KB ? (c < limit ? c - 1u : 0u) : few ? 0u : 1u;
+    partners += c - 1u; // below 2^26
+    paired += c > 1u && c <= 4u ? 1u : 0u;
   }
-  light = __reduce_add_sync(0xffffffffu, light);
-  heavy = __reduce_add_sync(0xffffffffu, heavy);
+  light    = __reduce_add_sync(0xffffffffu, light);
+  heavy    = __reduce_add_sync(0xffffffffu, heavy);
+  partners = __reduce_add_sync(0xffffffffu, partners);
+  paired   = __reduce_add_sync(0xffffffffu, paired);
   if (tid == 0)
   {
     heavy_sum = 0u;
@@ -201,12 +210,16 @@ __device__ __noinline__ void finish_sample(const HistogramParams& p, unsigned ch
   {
     atomicAdd(&light_sum, light);
     atomicAdd(&heavy_sum, heavy);
+    atomicAdd(&partners_sum, partners);
+    atomicAdd(&paired_sum, paired);
   }
   __syncthreads();
   if (tid == 0)
   {
     p.finish->light[level - 1] = light_sum;
     p.finish->heavy[level - 1] = heavy_sum;
+    p.finish->partners[level - 1] = partners_sum;
+    p.finish->paired[level - 1]   = paired_sum;
     finish_sampled<KB>(p);
   }
   __syncthreads(); // the shared memory is the histogram's again

@@ -129,6 +129,9 @@ struct FinishControl
   uint32_t done[FINISH_MAX_PHASES];
   uint32_t sampled_digits; // the choice when no digit is trivial
   uint32_t sampled_piece;
+  // of the sample, beside light and heavy (finish_choose)
+  uint32_t partners[MAX_PASSES];
+  uint32_t paired[MAX_PASSES];
 };
 
 struct HistogramParams

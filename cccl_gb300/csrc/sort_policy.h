@@ -366,8 +366,10 @@ static_assert(FINISH_SAMPLE_MOST < (1u << 14), "a slot counts in 14 bits");
 
 // Top digits to partition by (0: run every digit pass). `trivial_mask`: passes whose digit is
 // constant; light[l] and heavy[l]: what the sample of S keys found for the top l + 1 digits
-// (finish_sample; for whole keys: groups of two and three, and all small groups). The mean number of other keys in the bucket of a sampled key is n / S times
-// the mean number of other sampled keys in it. A candidate
+// (finish_sample; for whole keys: groups of two and three, and all small groups); partners[l] and
+// paired[l]: the other keys in the groups of all sampled keys, and the sampled keys in groups of two to
+// four. The mean number of other keys in the bucket of a sampled key is n / S times the mean number of
+// other sampled keys in it. A candidate
 //   * must leave buckets of at most 0.85 of the finish's capacity in that mean (up to 2.4 times
 //     the mean then fits its second launch);
 //   * must not crowd the finish's bins (FINISH_BIN_MAX): they split a piece 3328 or 3840 ways, so
@@ -382,7 +384,8 @@ static_assert(FINISH_SAMPLE_MOST < (1u << 14), "a slot counts in 14 bits");
 //     cluster at every scale, and the pieces would too.
 GB300_HD inline int finish_choose(int kb, uint32_t trivial_mask, const unsigned long long* light, const uint32_t* heavy,
                                   unsigned long long n, uint32_t samples, uint32_t cap, float cost, int plan_mode,
-                                  uint32_t* piece_items)
+                                  uint32_t* piece_items, const uint32_t* partners = nullptr,
+                                  const uint32_t* paired = nullptr)
 {
   int total = 0;
   for (int q = 0; q < kb; ++q)
@@ -424,6 +427,16 @@ GB300_HD inline int finish_choose(int kb, uint32_t trivial_mask, const unsigned 
     const float pairs = 0.5f * float(light[digits - 1]);
     const float below = 0.5f * (float(light[digits]) - float(heavy[kb - 1]));
     if (pairs >= 16.0f && heavy[digits - 1] < samples / 64u && digits < kb - 1 && below > pairs / 128.0f + 3.0f)
+    {
+      return 0;
+    }
+    // The same where some groups are large, as those of ANDs of two words are (21.5 M u64 pairs took 1.87 ms,
+    // 1.19 by all passes): of the other keys in a key's group, all groups counted, at most every 128th may
+    // still be with it a digit further down. What is counted there are the keys in groups of two to
+    // four, not pairs: one dense place (a clump, the lowest keys of a steep density) makes large
+    // groups, which the tail takes. A two-hundredth of the sample is let pass for small clumps.
+    if (partners != nullptr && heavy[digits - 1] < samples / 4u && digits < kb - 1
+        && float(paired[digits]) - float(paired[kb - 1]) > float(partners[digits - 1]) / 128.0f + float(samples) / 200.0f)
     {
       return 0;
     }
